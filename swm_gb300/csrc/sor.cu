@@ -7,32 +7,45 @@
 // sqrt(sum res^2) drops below eps (:213-218), max_count = 1000 max(Nx, Ny)
 // on a first call and 10 max(Nx, Ny) after it (:166-176).
 //
-// Layout: the coefficients, the right-hand side, chi and the ocean mask are
-// kept split by colour, row by row: cell (i, j) of colour (i + j) % 2 sits at
-// j * W + i / 2 of its colour's arrays (W = ceil(Nx / 2)).  A half-sweep then
-// reads only its own colour's coefficients, right-hand side, reciprocal
-// diagonal and chi (and the other colour's chi as neighbours): 10 words per
-// point and iteration, SOR_CELLS consecutive cells of the colour per thread,
-// coalesced.  Each cell's update is the reference's expression in the
-// reference's order (this file is compiled without FMA contraction), so chi
-// is bit for bit the restatement's when the iteration counts agree; within a
-// colour no cell reads another of its own colour (the periodic wrap only
-// pairs land cells, which stay fixed).
+// Layout: the right-hand side, chi and the masks are kept split by colour,
+// row by row: cell (i, j) of colour (i + j) % 2 sits at j * W + i / 2 of its
+// colour's arrays (W = ceil(Nx / 2)).  The coefficients depend on the row and
+// on the masks of the cell's four faces only, so a row keeps its three face
+// coefficients and the 16 diagonals its mask cases give, and a cell a byte of
+// mask bits: 33 B a point and iteration where one word per coefficient took
+// 80.  Each cell's update is the reference's expression in the reference's
+// order (this file is compiled without FMA contraction), so chi is bit for
+// bit the restatement's when the iteration counts agree; within a colour no
+// cell reads another of its own colour (the periodic wrap only pairs land
+// cells, which stay fixed).
 //
-// Division: GB300's FP64 rate is low and the half-sweep is bound by it, so
-// the update's division by the diagonal coefficient is formed from that
-// coefficient's reciprocal, set up once, by Markstein's correction
-// (div_rn below): the same correctly rounded quotient with five FP64
-// operations.
+// Division: GB300's FP64 rate is low (an FP64 warp instruction holds an SM's
+// pipe for 19 cycles) and a sweep is bound by it, so the division by the
+// diagonal is formed from its reciprocal in two words (divide.cuh): 16 FP64
+// operations a cell, 19 with the one-word reciprocal.
 //
-// Control: the relaxation factor, the iteration counter and the stop flag
-// live on the device.  Each half-sweep kernel sums res^2 per warp with
-// shuffles and per block; the last block to finish (fence and counter) adds
-// the blocks in a fixed order, advances the relaxation schedule, and after
-// the second colour applies the stop test.  The kernels take no per-
-// iteration arguments, so a batch of iterations is one CUDA graph, replayed
-// until the flag is set; kernels after convergence (or max_count) return at
-// once.  The host reads the flag once per batch.
+// Control: one cooperative launch runs a batch of iterations, one block per
+// SM.  Every block owns an equal, fixed span of cells of each colour (every
+// SM gets the same number of FP64 instructions) and publishes, after each
+// colour, how far it is; before a colour a block waits only for the blocks
+// whose cells are next to its own.  The relaxation schedule depends on the
+// iteration number alone.  The stop test is kept off that path: chi
+// alternates between two buffers, iteration l's norm is added by one warp of
+// every block (all in the same order, so all decide alike) while the others
+// run iteration l + 1 into the other buffer, and only iteration l + 2, which
+// would overwrite iteration l's chi, waits for the decision.  chi of other
+// blocks is read through L2.  Every wait is bounded: a thread that gives up
+// sets ctl->failed, which ends the waits of all others.
+//
+// One iteration, with a launch per colour and one-word reciprocals, and now:
+//   201 x 101 points      22.8 us ->   8.3 us  (waits and the FP64 latency chain)
+//   1025 x 769            47.0 us ->  32.3 us  (FP64 pipe 78 % busy; the 386 blocks of a
+//                                              colour left a last wave half empty)
+//   2049 x 2049            186 us ->   140 us  (FP64 pipe 95 % busy)
+// at 9.75 ns per FP64 warp instruction and SM, measured (19 cycles).  480
+// threads of four cells in flight against 992 of one: 15.6 against 17.1 us at
+// 513 x 513, the same from 1025 x 769 on.
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -42,56 +55,68 @@
 // device control block of a solve
 struct SorCtl {
   double relax;      // relaxation factor of the next half-sweep
-  double sum0;       // sum of res^2 of the current iteration's first colour
   double anorm;      // correction norm of the last finished iteration
   double eps;        // stop when the correction norm falls below it
-  int l;             // the iteration the next half-sweep belongs to (1-based)
+  int l;             // the next iteration (1-based)
   int max_count;
   int done;          // 1: converged (at iteration iters)
   int iters;
-  unsigned count;    // blocks finished in the running half-sweep
+  unsigned failed;   // a block gave up at the barrier
+};
+
+// one row's coefficients: 1/ax (zonal faces), cos_v / ay at the north and
+// south faces, and the diagonal by mask case (bit 0 east, 1 west, 2 north,
+// 3 south face open) with its reciprocal
+struct SorRow {
+  double a, n, s, pad;
+  swm::FixedDiv c4[16];
 };
 
 struct SorState {
-  double *c[5] = {};       // ElSolvSOR_c(:,:,1..5), natural layout (set-up only)
   double *chi = nullptr, *B = nullptr;   // natural layout; chi: calc_lib::chi, kept between
                                          // swm_gpu_nondivergent calls
   double *chi_io = nullptr;              // natural layout: elsolv_sor_gpu_solve's chi
-  double *cs[2][5] = {};   // coefficients split by colour
-  double *rc4[2] = {};     // 1 / ElSolvSOR_c(:,:,5), split by colour
-  uint8_t *ms[2] = {};     // ocean mask split by colour (0 also on the padding of odd rows)
-  int *bad = nullptr;      // set-up: 1 when an ocean cell's diagonal is outside div_rn's range
-  bool fast = true;        // every ocean diagonal inside div_rn's range
-  double *Bs[2] = {}, *chis[2] = {};     // right-hand side and chi split by colour
-  double *partial = nullptr;   // per-block sums of res^2 of a half-sweep
+  SorRow *rows = nullptr;
+  uint8_t *ms[2] = {};     // mask bits split by colour: 0-3 open faces, 4 ocean (0 on the padding of odd rows)
+  double *Bs[2] = {};          // right-hand side split by colour
+  double *chis[2][2] = {};     // chi split by colour: [iteration & 1][colour]
+  double *partial = nullptr;   // per-block sums of res^2 of the last SOR_PART iterations
   SorCtl *ctl = nullptr;
+  unsigned *flags = nullptr;   // per block: half-sweeps of the running batch that it has finished, then
+                               // per block: iterations whose sums it has stored
   double *und = nullptr, *vnd = nullptr;  // non-divergent flow
-  int W = 0, nblocks = 0;      // split row length; blocks of a half-sweep
-  cudaGraphExec_t graph = nullptr;  // SOR_BATCH iterations
+  int W = 0;                   // split row length
+  unsigned span = 0;           // cells of a colour per block
+  int blocks = 0, threads = 0; // of a batch; the last warp adds the norms
 };
 
-constexpr int SOR_THREADS = 256;
-constexpr int SOR_CELLS = 4;  // consecutive cells of the colour per thread (one 32-bit word of mask bytes)
-constexpr int SOR_BATCH = 32;  // iterations per graph replay (one host read of the flag)
+constexpr int SOR_CELL_THREADS = 480;  // most threads of a block that own cells
+constexpr int SOR_CELLS = 4;           // cells whose loads a thread has in flight
+// kept norms: a block that starts adding iteration l + 3's has decided l + 1,
+// for which every block has started l + 2 and so decided l
+constexpr int SOR_PART = 4;            // (also the relaxation factors' ring)
+constexpr unsigned long long SOR_WAIT_NS = 2000000000ull;  // a wait that has not ended after 2 s
 
 namespace swm {
 
-__global__ void k_sor_coeff(Dev d, SorState s) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= d.nx || j >= d.ny) return;
-  size_t k = i + (size_t)d.nx * j;
-  int ip = i + 1 == d.nx ? 0 : i + 1, jp = j + 1 == d.ny ? 0 : j + 1;
-  size_t ki = ip + (size_t)d.nx * j, kj = i + (size_t)d.nx * jp;
-  const int8_t *oU = d.ocean[GU], *oV = d.ocean[GV];
+// init_ElSolv_SOR (:54-62), the coefficients of one row by the reference's
+// expressions
+__global__ void k_sor_rows(Dev d, SorRow *rows) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, j = t >> 4, q = t & 15;
+  if (j >= d.ny) return;
+  const int jp = j + 1 == d.ny ? 0 : j + 1;
   const double *cE = d.cosl[GE], *cV = d.cosl[GV];
-  double A = d.A, dL = d.dLambda, dT = d.dTheta;
-  double ax = (A * cE[j] * dL) * (A * cE[j] * dL);
-  double ay = (A * A * cE[j] * (dT * dT));
-  s.c[0][k] = oU[ki] / ax;
-  s.c[1][k] = oU[k] / ax;
-  s.c[2][k] = cV[jp] * oV[kj] / ay;
-  s.c[3][k] = cV[j] * oV[k] / ay;
-  s.c[4][k] = (-oU[ki] - oU[k]) / ax + (-cV[jp] * oV[kj] - cV[j] * oV[k]) / ay;
+  const double A = d.A, dL = d.dLambda, dT = d.dTheta;
+  const double ax = (A * cE[j] * dL) * (A * cE[j] * dL);
+  const double ay = (A * A * cE[j] * (dT * dT));
+  const int e = q & 1, w = (q >> 1) & 1, n = (q >> 2) & 1, s = (q >> 3) & 1;
+  SorRow &R = rows[j];
+  if (q == 0) {
+    R.a = 1 / ax;
+    R.n = cV[jp] / ay;
+    R.s = cV[j] / ay;
+  }
+  R.c4[q] = fixed_div((-e - w) / ax + (-cV[jp] * n - cV[j] * s) / ay);
 }
 
 // natural <-> colour-split layout (join 0: natural -> split, 1: split -> natural)
@@ -105,102 +130,231 @@ __global__ void k_sor_split(double *nat, double *s0, double *s1, int nx, int ny,
   else sp[q] = nat[k];
 }
 
-// set-up: the reciprocal diagonal and the split ocean mask of colour col;
-// *bad = 1 when an ocean cell's diagonal is outside div_rn's range
-__global__ void k_sor_recip(const int8_t *__restrict__ ocean, const double *__restrict__ c4, double *__restrict__ rc4,
-                            uint8_t *__restrict__ ms, int nx, int ny, int W, int col, int *bad) {
+// set-up: the split mask bits of colour col
+__global__ void k_sor_mask(Dev d, uint8_t *__restrict__ ms, int W, int col) {
   const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (size_t)W * ny) return;
+  if (q >= (size_t)W * d.ny) return;
   const int j = (int)(q / W), i = 2 * (int)(q % W) + ((col + j) & 1);
-  const bool o = i < nx && ocean[i + (size_t)nx * j] != 0;
-  ms[q] = o;
-  rc4[q] = 1. / c4[q];
-  if (o && !div_rn_range(c4[q])) atomicOr(bad, 1);
+  unsigned m = 0;
+  if (i < d.nx) {
+    const int ip = i + 1 == d.nx ? 0 : i + 1, jp = j + 1 == d.ny ? 0 : j + 1;
+    const size_t k = i + (size_t)d.nx * j;
+    const int8_t *oU = d.ocean[GU], *oV = d.ocean[GV];
+    m = (oU[ip + (size_t)d.nx * j] != 0) | (oU[k] != 0) << 1 | (oV[i + (size_t)d.nx * jp] != 0) << 2 |
+        (oV[k] != 0) << 3 | (d.ocean[GE][k] != 0) << 4;
+  }
+  ms[q] = (uint8_t)m;
 }
 
-// One half-sweep of colour col (0: (i+j) even in 0-based indices, the
-// reference's colour 1) over the colour-split arrays, SOR_CELLS cells per
-// thread; then the block sums of res^2 and, in the last block, the
-// iteration's bookkeeping.  FAST: the division by div_rn (every ocean
-// diagonal in its range; a numerator outside it still divides).
-template <bool FAST>
-__global__ void __launch_bounds__(SOR_THREADS) k_sor_half(SorState s, int nx, int ny, int col, double rJ) {
+// Bounded wait: until ready() holds.  False when the wait ran out or another
+// thread's did (ctl->failed).
+// SLEEP: nanoseconds between looks, for waits that are not urgent.
+template <int SLEEP = 0, typename F>
+__device__ __forceinline__ bool sor_wait(SorCtl *ctl, F ready) {
+  unsigned long long t0 = 0;
+  for (unsigned spins = 1;; spins++) {
+    if (ready()) return true;
+    if (SLEEP) __nanosleep(SLEEP);
+    if ((spins & 1023u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      if (t - t0 > SOR_WAIT_NS) atomicExch(&ctl->failed, 1u);
+      if (*(volatile unsigned *)&ctl->failed) return false;
+    }
+  }
+}
+
+__device__ __forceinline__ unsigned sor_flag(const unsigned *f) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+  return v;
+}
+// (with the block's writes before the last barrier)
+__device__ __forceinline__ void sor_publish(unsigned *f, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(f), "r"(v) : "memory");
+}
+
+// Iterations ctl->l .. of the solve, at most niter of them: colour 0 ((i+j)
+// even in 0-based indices, the reference's colour 1), then colour 1, until
+// the correction norm falls below eps or max_count is reached.  Cooperative
+// launch of s.blocks blocks; block b owns cells [b * span, (b + 1) * span) of
+// each colour.  FP64-pipe bound.
+__global__ void __launch_bounds__(SOR_CELL_THREADS + 32, 1) k_sor_batch(SorState s, int nx, int ny, double rJ,
+                                                                        int niter) {
   SorCtl *ctl = s.ctl;
-  if (ctl->done || ctl->l > ctl->max_count) return;  // converged, or max_count reached
-  const double relax = ctl->relax;
-  const int W = s.W;
-  const size_t ns = (size_t)W * ny;
-  const size_t q0 = ((size_t)blockIdx.x * SOR_THREADS + threadIdx.x) * SOR_CELLS;
-  const double *const *cs = s.cs[col];
-  double *x = s.chis[col];
-  double r2 = 0.;
-  if (q0 < ns) {
-    uint32_t m4 = 0;  // the cells' mask bytes
-    if (q0 + SOR_CELLS <= ns) {
-      m4 = *reinterpret_cast<const uint32_t *>(s.ms[col] + q0);
-    } else {
-      for (int k = 0; k < SOR_CELLS && q0 + k < ns; k++) m4 |= (uint32_t)s.ms[col][q0 + k] << (8 * k);
+  __shared__ double buf[2][SOR_CELL_THREADS];  // res^2 by thread, of even and odd iterations
+  __shared__ double relax[SOR_PART][2];        // factors of the iterations up to decided + 2
+  __shared__ volatile int swept;    // the last iteration whose cells are done
+  __shared__ volatile int decided;  // the last iteration whose norm is known,
+  __shared__ volatile int stop;     // and the one that met the stop test
+  __shared__ int go, fail;
+  const int l0 = ctl->l, lend = min(l0 + niter - 1, ctl->max_count);
+  if (ctl->done || ctl->failed || l0 > lend) return;  // the same in every block: nobody has written yet
+  const unsigned W = s.W, ns = W * (unsigned)ny, G = gridDim.x, blk = blockIdx.x, span = s.span;
+  const unsigned q0 = blk * span, q1 = min(q0 + span, ns);
+  const unsigned tid = threadIdx.x, T = blockDim.x - 32;  // threads that own cells
+  const double eps = ctl->eps;
+  double r = ctl->relax;  // the factor of the next half-sweep
+  // the schedule of main_ElSolv_SOR (:206-210): after the first colour of the
+  // first iteration 1 / (1 - rJ^2 / 2), else 1 / (1 - rJ^2 relax / 4)
+  auto schedule = [&](int l) {
+    for (int col = 0; col < 2; col++) {
+      relax[l % SOR_PART][col] = r;
+      r = 1. / (1. - (col == 0 && l == 1 ? .5 * rJ * rJ : .25 * rJ * rJ * r));
     }
-#pragma unroll
-    for (int k = 0; k < SOR_CELLS; k++) {
-      if (!((m4 >> (8 * k)) & 0xffu)) continue;
-      const size_t q = q0 + k;
-      const int j = (int)(q / W), i = 2 * (int)(q - (size_t)j * W) + ((col + j) & 1);
-      const int ip = i + 1 == nx ? 0 : i + 1, im = i == 0 ? nx - 1 : i - 1;
-      const int jp = j + 1 == ny ? 0 : j + 1, jm = j == 0 ? ny - 1 : j - 1;
-      // neighbours are of the other colour except across an odd periodic wrap
-      auto at = [&](int a, int b) { return s.chis[(a + b) & 1][(size_t)b * W + (a >> 1)]; };
-      const double c4 = cs[4][q];
-      const double num = relax * (cs[0][q] * at(ip, j) + cs[1][q] * at(im, j) + cs[2][q] * at(i, jp) +
-                                  cs[3][q] * at(i, jm) + c4 * x[q] - s.Bs[col][q]);
-      const double res = FAST && div_rn_range(num) ? div_rn(num, c4, s.rc4[col][q]) : num / c4;
-      x[q] = x[q] - res;
-      r2 = r2 + res * res;
-    }
-  }
-  // block sum: shuffles within warps, then the warps in order
-  __shared__ double wsum[SOR_THREADS / 32];
-  __shared__ bool last;
-  for (int o = 16; o > 0; o >>= 1) r2 += __shfl_down_sync(0xffffffffu, r2, o);
-  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = r2;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0.;
-    for (int w = 0; w < SOR_THREADS / 32; w++) b += wsum[w];
-    s.partial[blockIdx.x] = b;
-    __threadfence();
-    last = atomicAdd(&ctl->count, 1u) == gridDim.x - 1;
+  };
+  if (tid == T) {
+    swept = decided = l0 - 1;
+    stop = 0x7fffffff;
+    fail = 0;
+    schedule(l0);
+    schedule(l0 + 1);
   }
   __syncthreads();
-  if (!last) return;
-  // last block: the blocks' sums in block order (thread t adds blocks t,
-  // t + 256, ..., then the warps' shuffle trees, then the warps in order)
-  __threadfence();
-  double v = 0.;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += SOR_THREADS) v += ((volatile double *)s.partial)[b];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.;
-    for (int w = 0; w < SOR_THREADS / 32; w++) tot += wsum[w];
-    const int l = ctl->l;
-    // the schedule of main_ElSolv_SOR (:206-210): after the first colour of
-    // the first iteration 1 / (1 - rJ^2 / 2), else 1 / (1 - rJ^2 relax / 4)
-    if (col == 0 && l == 1) ctl->relax = 1. / (1. - .5 * rJ * rJ);
-    else ctl->relax = 1. / (1. - .25 * rJ * rJ * relax);
-    if (col == 0) {
-      ctl->sum0 = tot;
-    } else {
-      const double an = sqrt(ctl->sum0 + tot);
-      ctl->anorm = an;
-      if (an < ctl->eps) {
-        ctl->done = 1;
-        ctl->iters = l;
+
+  if (tid >= T) {  // the norms and the schedule
+    const unsigned lane = tid - T;
+    // a total above eps^2 by more than rounding needs no root
+    const double far2 = eps * eps * (1. + 1e-12) + 1e-300;
+    unsigned *stored = s.flags + G;
+    double v = 0.;
+    int l = l0;
+    bool ok = true, met = false;
+    for (; l <= lend && !met; l++) {
+      ok = sor_wait(ctl, [&]() { return swept >= l; });
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      __threadfence_block();
+      // the block's sum, then the blocks', each in a fixed order
+      v = 0.;
+      for (unsigned k = lane; k < T; k += 32) v += buf[l & 1][k];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      double *part = s.partial + (size_t)(l % SOR_PART) * G;
+      if (lane == 0) {
+        part[blk] = v;
+        sor_publish(stored + blk, (unsigned)(l - l0) + 1u);
+        schedule(l + 2);
       }
-      ctl->l = l + 1;
+      __syncwarp();
+      for (unsigned b = lane; b < G && ok; b += 32)
+        ok = sor_wait<20>(ctl, [&]() { return sor_flag(stored + b) >= (unsigned)(l - l0) + 1u; });
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      v = 0.;
+      for (unsigned b = lane; b < G; b += 32) v += __ldcg(part + b);
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      met = v < far2 && sqrt(v) < eps;
+      if (lane == 0) {
+        if (met) stop = l;
+        __threadfence_block();
+        decided = l;
+      }
+      __syncwarp();
     }
-    ctl->count = 0;
+    if (ok && blk == 0 && lane == 0) {
+      ctl->anorm = sqrt(v);
+      ctl->relax = relax[l % SOR_PART][0];
+      ctl->l = l;
+      if (met) {
+        ctl->iters = l - 1;
+        ctl->done = 1;
+      }
+    }
+    return;
+  }
+
+  // blocks whose cells are next to this block's: those of the W + 1 cells
+  // before and after the span (rows wrap)
+  unsigned first = 0, near = G;  // near blocks, from block `first` on
+  if (2 * (W + 1) + 2 * span < ns) {
+    first = ((q0 + ns - (W + 1)) % ns) / span;
+    near = ((q1 + W) % ns / span + G - first) % G + 1;
+  }
+  double r2 = 0.;
+  unsigned h = 0;  // half-sweeps done
+  for (int l = l0; l <= lend; l++) {
+    for (int col = 0; col < 2; col++, h++) {
+      // the neighbours have finished the half-sweep before this one, and
+      // before iteration l overwrites it, iteration l - 2 is known not to be the last
+      bool ok = true;
+      if (h)
+        for (unsigned t = tid; t < near && ok; t += T) {
+          const unsigned b = (first + t) % G;
+          if (b != blk) ok = sor_wait(ctl, [&]() { return sor_flag(s.flags + b) >= h; });
+        }
+      if (tid == 0 && col == 0) {
+        ok = ok && sor_wait(ctl, [&]() { return decided >= l - 2; });
+        __threadfence_block();
+        go = stop > l - 2;
+      }
+      if (!ok) fail = 1;
+      __syncwarp();
+      asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
+      if (fail) return;
+      if (col == 0 && !go) return;
+      const double rel = relax[l % SOR_PART][col];
+      const double *x = s.chis[(l - 1) & 1][col], *Bc = s.Bs[col];
+      const double *y = s.chis[(l - 1 + col) & 1][col ^ 1];  // colour 1 reads this iteration's colour 0
+      double *xn = s.chis[l & 1][col];
+      const uint8_t *ms = s.ms[col];
+      for (unsigned qb = q0 + tid; qb < q1; qb += SOR_CELLS * T) {
+        unsigned m[SOR_CELLS], jj[SOR_CELLS];
+        double xq[SOR_CELLS], b[SOR_CELLS], ve[SOR_CELLS], vw[SOR_CELLS], vn[SOR_CELLS], vs[SOR_CELLS];
+#pragma unroll
+        for (int u = 0; u < SOR_CELLS; u++) {
+          const unsigned q = qb + u * T;
+          m[u] = q < q1 ? ms[q] : 0u;
+          if (!(m[u] & 16u)) continue;
+          const unsigned j = q / W, c = q - j * W, par = (col + j) & 1;
+          const int i = 2 * (int)c + (int)par;
+          jj[u] = j;
+          xq[u] = x[q];
+          b[u] = Bc[q];
+          if (i > 0 && i + 1 < nx && j > 0 && (int)j + 1 < ny) {
+            // the four neighbours are of the other colour
+            ve[u] = __ldcg(y + q + par);
+            vw[u] = __ldcg(y + q + par - 1);
+            vn[u] = __ldcg(y + q + W);
+            vs[u] = __ldcg(y + q - W);
+          } else {  // the frame: periodic neighbours, of this cell's own colour across an odd wrap
+            const int ip = i + 1 == nx ? 0 : i + 1, im = i == 0 ? nx - 1 : i - 1;
+            const int jp = (int)j + 1 == ny ? 0 : (int)j + 1, jm = j == 0 ? ny - 1 : (int)j - 1;
+            auto at = [&](int a, int bb) {
+              const int k = (a + bb) & 1;
+              return __ldcg((k == col ? x : y) + (size_t)bb * W + (a >> 1));
+            };
+            ve[u] = at(ip, (int)j);
+            vw[u] = at(im, (int)j);
+            vn[u] = at(i, jp);
+            vs[u] = at(i, jm);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < SOR_CELLS; u++) {
+          if (!(m[u] & 16u)) continue;
+          const SorRow &R = s.rows[jj[u]];
+          const double ce = m[u] & 1u ? R.a : 0., cw = m[u] & 2u ? R.a : 0.;
+          const double cn = m[u] & 4u ? R.n : 0., cs = m[u] & 8u ? R.s : 0.;
+          const FixedDiv &D = R.c4[m[u] & 15u];
+          const double num = rel * (ce * ve[u] + cw * vw[u] + cn * vn[u] + cs * vs[u] + D.b * xq[u] - b[u]);
+          const double res = div_fixed(num, D);
+          xn[qb + u * T] = xq[u] - res;
+          r2 = r2 + res * res;
+        }
+      }
+      if (col == 1) buf[l & 1][tid] = r2;
+      __syncwarp();
+      asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
+      if (tid == 0) {
+        sor_publish(s.flags + blk, h + 1);
+        if (col == 1) {
+          __threadfence_block();
+          swept = l;
+        }
+      }
+    }
+    r2 = 0.;
   }
 }
 
@@ -280,6 +434,21 @@ __global__ void k_div_check(int64_t n, uint64_t seed, unsigned long long *bad) {
     const double q = __ddiv_rn(a, b), y = __ddiv_rn(1., b), f = div_fast(a, b, y);
     const bool same = __double_as_longlong(f) == __double_as_longlong(q) || (q != q && f != f);
     mism += !same;
+    // the two-word reciprocal: this numerator, and the two numerators whose
+    // quotients come closest to a midpoint of two doubles
+    const FixedDiv D = fixed_div(b);
+    double g = div_fixed(a, D);
+    mism += !(__double_as_longlong(g) == __double_as_longlong(q) || (q != q && g != g));
+    const unsigned long long one = 1ull << 52, B = ((unsigned long long)__double_as_longlong(b) & (one - 1)) | one;
+    if (B & 1) {
+      unsigned long long x = 1;
+      for (int t = 0; t < 54; t++) x = (x & 1) ? (x + B) >> 1 : x >> 1;
+      for (int t = 0; t < 2; t++, x = B - x) {
+        if (x < one) continue;
+        const double w = __longlong_as_double((long long)((1023ull << 52) | (x & (one - 1))));
+        mism += __double_as_longlong(div_fixed(w, D)) != __double_as_longlong(__ddiv_rn(w, b));
+      }
+    }
   }
   for (int o = 16; o > 0; o >>= 1) mism += __shfl_down_sync(0xffffffffu, mism, o);
   if ((threadIdx.x & 31) == 0 && mism) atomicAdd(bad, mism);
@@ -288,16 +457,13 @@ __global__ void k_div_check(int64_t n, uint64_t seed, unsigned long long *bad) {
 void sor_free(swm_gpu_ctx *c) {
   if (!c->sor) return;
   SorState *s = c->sor;
-  if (s->graph) cudaGraphExecDestroy(s->graph);
-  for (int q = 0; q < 5; q++) cudaFree(s->c[q]);
   for (int col = 0; col < 2; col++) {
-    for (int q = 0; q < 5; q++) cudaFree(s->cs[col][q]);
     cudaFree(s->Bs[col]);
-    cudaFree(s->chis[col]);
-    cudaFree(s->rc4[col]);
+    cudaFree(s->chis[0][col]);
+    cudaFree(s->chis[1][col]);
     cudaFree(s->ms[col]);
   }
-  cudaFree(s->bad);
+  cudaFree(s->rows); cudaFree(s->flags);
   cudaFree(s->chi); cudaFree(s->chi_io); cudaFree(s->B); cudaFree(s->partial); cudaFree(s->ctl);
   cudaFree(s->und); cudaFree(s->vnd);
   delete s;
@@ -313,81 +479,47 @@ extern "C" {
 int elsolv_sor_gpu_init(swm_gpu_ctx *c) {
   SWM_ON_DEVICE(c ? c->device : -1);
   SWM_REQUIRE(c && c->stage >= 1, "elsolv_sor_gpu_init: call after swm_gpu_domain");
+  const size_t n = c->n;
+  const int W = (c->nx + 1) / 2;
+  const size_t ns = (size_t)W * c->ny;
+  SWM_REQUIRE(ns < (1ull << 31), "elsolv_sor_gpu_init: grid too large");
   sor_free(c);
   SorState *s = new SorState();
   c->sor = s;
-  const size_t n = c->n;
-  s->W = (c->nx + 1) / 2;
-  const size_t ns = (size_t)s->W * c->ny;
-  s->nblocks = (int)((ns + (size_t)SOR_THREADS * SOR_CELLS - 1) / ((size_t)SOR_THREADS * SOR_CELLS));
-  for (int q = 0; q < 5; q++) SWM_CK(cudaMalloc((void **)&s->c[q], n * 8));
+  s->W = W;
+  int sms = 0;
+  SWM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device < 0 ? 0 : c->device));
+  // one block per SM, of no more threads than cells of a colour (and the warp
+  // that adds the norms)
+  s->span = (unsigned)std::max<size_t>(32, (ns + sms - 1) / sms);
+  s->blocks = (int)((ns + s->span - 1) / s->span);
+  s->threads = (int)std::min<size_t>(SOR_CELL_THREADS, ((size_t)s->span + 31) / 32 * 32) + 32;
+  SWM_CK(cudaMalloc((void **)&s->rows, (size_t)c->ny * sizeof(SorRow)));
   for (int col = 0; col < 2; col++) {
-    for (int q = 0; q < 5; q++) SWM_CK(cudaMalloc((void **)&s->cs[col][q], ns * 8));
     SWM_CK(cudaMalloc((void **)&s->Bs[col], ns * 8));
-    SWM_CK(cudaMalloc((void **)&s->chis[col], ns * 8));
-    SWM_CK(cudaMalloc((void **)&s->rc4[col], ns * 8));
-    SWM_CK(cudaMalloc((void **)&s->ms[col], ns + SOR_CELLS));
+    SWM_CK(cudaMalloc((void **)&s->chis[0][col], ns * 8));
+    SWM_CK(cudaMalloc((void **)&s->chis[1][col], ns * 8));
+    SWM_CK(cudaMalloc((void **)&s->ms[col], ns));
   }
-  SWM_CK(cudaMalloc((void **)&s->bad, sizeof(int)));
-  SWM_CK(cudaMemsetAsync(s->bad, 0, sizeof(int), c->stream));
   SWM_CK(cudaMalloc((void **)&s->chi, n * 8));
   SWM_CK(cudaMalloc((void **)&s->chi_io, n * 8));
   SWM_CK(cudaMalloc((void **)&s->B, n * 8));
-  SWM_CK(cudaMalloc((void **)&s->partial, (size_t)s->nblocks * 8));
+  SWM_CK(cudaMalloc((void **)&s->partial, (size_t)SOR_PART * s->blocks * 8));
   SWM_CK(cudaMalloc((void **)&s->ctl, sizeof(SorCtl)));
+  SWM_CK(cudaMalloc((void **)&s->flags, 2 * s->blocks * sizeof(unsigned)));
   SWM_CK(cudaMemsetAsync(s->ctl, 0, sizeof(SorCtl), c->stream));
   SWM_CK(cudaMemsetAsync(s->chi, 0, n * 8, c->stream));  // calc_lib::chi starts at 0
-  dim3 b(32, 8), g((c->nx + 31) / 32, (c->ny + 7) / 8);
-  k_sor_coeff<<<g, b, 0, c->stream>>>(c->dev(), *s);
-  const unsigned nb = (unsigned)((n + 255) / 256);
-  for (int q = 0; q < 5; q++)
-    k_sor_split<<<nb, 256, 0, c->stream>>>(s->c[q], s->cs[0][q], s->cs[1][q], c->nx, c->ny, s->W, 0);
-  const unsigned nbs = (unsigned)((ns + 255) / 256);
+  const Dev d = c->dev();
+  k_sor_rows<<<(16 * c->ny + 127) / 128, 128, 0, c->stream>>>(d, s->rows);
   for (int col = 0; col < 2; col++)
-    k_sor_recip<<<nbs, 256, 0, c->stream>>>(c->d_ocean[GE], s->cs[col][4], s->rc4[col], s->ms[col], c->nx, c->ny,
-                                            s->W, col, s->bad);
-  c->launches += 8;
+    k_sor_mask<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(d, s->ms[col], W, col);
+  c->launches += 3;
   SWM_CK(cudaGetLastError());
-  int bad = 0;
-  SWM_CK(cudaMemcpyAsync(&bad, s->bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   SWM_CK(cudaStreamSynchronize(c->stream));
-  s->fast = bad == 0;
   return SWM_GPU_OK;
 }
 
 }  // extern "C"
-
-namespace {
-
-// the two half-sweeps of one iteration
-void sor_iteration(swm_gpu_ctx *c, SorState *s) {
-  const double rJ = (double)(float)9.9999178e-1;  // default-real literal (ElSolv_SOR.f90:175)
-  for (int col = 0; col < 2; col++) {
-    if (s->fast) k_sor_half<true><<<s->nblocks, SOR_THREADS, 0, c->stream>>>(*s, c->nx, c->ny, col, rJ);
-    else k_sor_half<false><<<s->nblocks, SOR_THREADS, 0, c->stream>>>(*s, c->nx, c->ny, col, rJ);
-  }
-}
-
-// SOR_BATCH iterations as one graph, captured once per set-up (the kernels
-// read their iteration state and eps from the control block, so one capture
-// serves every batch and every call)
-int sor_graph(swm_gpu_ctx *c, SorState *s) {
-  if (s->graph) return SWM_GPU_OK;
-  SWM_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  for (int l = 0; l < SOR_BATCH; l++) sor_iteration(c, s);
-  cudaGraph_t g = nullptr;
-  SWM_CK(cudaStreamEndCapture(c->stream, &g));
-  cudaError_t e = cudaGraphInstantiate(&s->graph, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    s->graph = nullptr;
-    set_error(std::string("elsolv_sor_gpu_solve: cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    return SWM_GPU_ECUDA;
-  }
-  return SWM_GPU_OK;
-}
-
-}  // namespace
 
 // main_ElSolv_SOR on the device arrays s->B (right-hand side) and chi
 // (first guess in, solution out), natural layout; returns
@@ -398,24 +530,34 @@ static int sor_solve_device(swm_gpu_ctx *c, double *chi, double eps, int first_g
   const int max_count = first_guess ? (int)lround(1000. * mx) : (int)lround(10. * mx);
   const unsigned nb = (unsigned)((c->n + 255) / 256);
   k_sor_split<<<nb, 256, 0, c->stream>>>(s->B, s->Bs[0], s->Bs[1], c->nx, c->ny, s->W, 0);
-  k_sor_split<<<nb, 256, 0, c->stream>>>(chi, s->chis[0], s->chis[1], c->nx, c->ny, s->W, 0);
-  c->launches += 2;
+  for (int b = 0; b < 2; b++)  // both buffers: the sweeps leave land as it is
+    k_sor_split<<<nb, 256, 0, c->stream>>>(chi, s->chis[b][0], s->chis[b][1], c->nx, c->ny, s->W, 0);
+  c->launches += 3;
   SorCtl ctl = {};
   ctl.relax = 1.;
   ctl.l = 1;
   ctl.max_count = max_count;
   ctl.eps = eps;
   SWM_CK(cudaMemcpyAsync(s->ctl, &ctl, sizeof(SorCtl), cudaMemcpyHostToDevice, c->stream));
-  int rc = sor_graph(c, s);
-  if (rc != SWM_GPU_OK) return rc;
-  for (int l = 1; l <= max_count; l += SOR_BATCH) {
-    SWM_CK(cudaGraphLaunch(s->graph, c->stream));
-    c->launches += 2 * SOR_BATCH;
+  double rJ = (double)(float)9.9999178e-1;  // default-real literal (ElSolv_SOR.f90:175)
+  int nx = c->nx, ny = c->ny;
+  // iterations of a batch: some tens of milliseconds at 4e10 cells a second
+  int batch = (int)std::min(4096., std::max(16., 1e9 / (double)c->n));
+  void *args[] = {s, &nx, &ny, &rJ, &batch};
+  for (int l = 1; l <= max_count; l += batch) {
+    SWM_CK(cudaMemsetAsync(s->flags, 0, 2 * s->blocks * sizeof(unsigned), c->stream));
+    SWM_CK(cudaLaunchCooperativeKernel((const void *)k_sor_batch, dim3(s->blocks), dim3(s->threads), args, 0, c->stream));
+    c->launches++;
     SWM_CK(cudaMemcpyAsync(&ctl, s->ctl, sizeof(SorCtl), cudaMemcpyDeviceToHost, c->stream));
     SWM_CK(cudaStreamSynchronize(c->stream));
+    if (ctl.failed) {
+      set_error("elsolv_sor_gpu_solve: a block waited too long for the others");
+      return SWM_GPU_EDEVICE;
+    }
     if (ctl.done) break;
   }
-  k_sor_split<<<nb, 256, 0, c->stream>>>(chi, s->chis[0], s->chis[1], c->nx, c->ny, s->W, 1);
+  const int last = (ctl.done ? ctl.iters : max_count) & 1;  // the buffer of the last iteration
+  k_sor_split<<<nb, 256, 0, c->stream>>>(chi, s->chis[last][0], s->chis[last][1], c->nx, c->ny, s->W, 1);
   c->launches++;
   SWM_CK(cudaGetLastError());
   if (anorm) *anorm = ctl.anorm;
