@@ -43,7 +43,7 @@ enum { SWM_MIX_LAPLACE = 0, SWM_MIX_BIHARMONIC = 1 /* project extension */ };
 /* ---- execution paths ---- */
 enum {
   SWM_PATH_PLAIN_FP64 = 0,    /* per-module FP64 kernels, bit-for-bit with the FP64 restatement */
-  SWM_PATH_FUSED_FP64 = 1,    /* one fused FP64 stencil kernel per step            */
+  SWM_PATH_FUSED_FP64 = 1,    /* FP64, every quantity formed once a step           */
   SWM_PATH_FUSED_FP32C = 2    /* fused FP32 stencil, state kept as FP32 hi+lo pair */
 };
 

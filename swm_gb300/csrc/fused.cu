@@ -1,281 +1,15 @@
-// fused.cu -- one-kernel-per-step SWM update (FULLY_NONLINEAR,
-// LINEARISED_STATE_OF_REST and no-linearisation modes).
-//
-// A CTA owns a TX x TY tile of cells.  It stages u, v, eta, the land/ocean
-// mask code and the depth for the tile plus an H-cell halo (H = 1 for the
-// reference's Laplacian-type stress, 2 for the biharmonic extension) in
-// shared memory, rebuilds every per-step diagnostic the reference keeps in
-// global arrays (D, Du/Dv/Dh, mass fluxes, vorticity, PV, Bernoulli,
-// P_lambda-lambda / P_lambda-theta) inside the tile, and writes only the new
-// state and the newest Adams-Bashforth increment.  Per cell and step the
-// kernel therefore moves the state in and out once, reads the two older
-// increments and writes the newest one -- the algorithmic minimum.
-//
-// T = double: the FP64 fused path.  (The FP32 compensated path is the row
-// marching kernel of march.cu.)
-//
-// Arithmetic follows the reference formulas (swm_nonlinear_timestep_module.f90
-// :182-449, swm_lateralmixing_module.f90:66-240, time_integration_module.f90
-// :74-112) with divisions by grid metrics replaced by per-row reciprocals, so
-// results agree with the FP64 restatement to rounding, not bit for bit.
+// fused.cu -- the fused paths' state: set-up, forcing that changes every step,
+// parameter blocks of the step kernels (FP64: fused64.cu; FP32 pairs:
+// march.cu), and the domain integrals.
 #include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
 #include "ctx.h"
 #include "fused32.h"
+#include "fused64.h"
 
 namespace swm {
-
-enum {
-  R_CE, R_CV, R_CU, R_FH, R_RE_DL, R_RE_DT, R_RU_DL, R_RV_DL, R_RH_DL, R_INV_CH,
-  R_PC0, R_HC0, R_TE, R_TH, R_TU, R_TV, R_NR
-};
-
-template <typename T>
-struct FP {
-  int nx, ny, mode, mix, qbf, barotropic, has_F, impl_uniform, gsq_uniform, wind_x, wind_y, wind_rows, tstep;
-  T dt, G, minD, lbc, q1, ts_rho, Ah, bih, eps;
-  T ab0, ab1, ab2;
-  T impl_s[3], gsq_s[2];
-  const uint8_t *mc;
-  const T *He, *rows, *Hu, *Hv;
-  const T *impl[3], *gsq[2];
-  const T *Fx, *Fy, *Fe;
-  const T *wx, *wy;
-  const T *u0, *v0, *e0;
-  T *u1, *v1, *e1;
-  const T *Gu1, *Gu2, *Gv1, *Gv2, *Ge1, *Ge2;
-  T *Gu3, *Gv3, *Ge3;
-};
-
-constexpr int TX = 32, TY = 8, NT = TX * TY;
-
-__device__ __forceinline__ int wrapi(int g, int n) {
-  if (g < 0) g += n;
-  if (g >= n) g -= n;
-  if (g >= n) g -= n;
-  return g;
-}
-
-template <typename T>
-__device__ __forceinline__ T recip_cnt(int c) {
-  // 1 / max(c, 1) for the mask-normalised interpolation weights
-  return c <= 1 ? T(1) : (c == 2 ? T(0.5) : (c == 3 ? T(1) / T(3) : T(0.25)));
-}
-
-template <typename T, int HALO>
-__global__ void __launch_bounds__(NT) k_fused(FP<T> p) {
-  constexpr int W = TX + 2 * HALO, HH = TY + 2 * HALO, NS = W * HH;
-  __shared__ T sU[NS], sV[NS], sE[NS], sD[NS], sMU[NS], sMV[NS], sPOT[NS], sB[NS], sPLL[NS], sPLT[NS];
-  __shared__ T sLU[HALO == 2 ? NS : 1], sLV[HALO == 2 ? NS : 1];
-  __shared__ uint8_t sM[NS];
-  const int tid = threadIdx.x;
-  const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
-  const int nx = p.nx, ny = p.ny;
-  const bool nl = p.mode == SWM_MODE_NONLINEAR;
-  auto S = [](int i, int j) { return (j + HALO) * W + (i + HALO); };
-  auto row = [&](int j) { return p.rows + (size_t)wrapi(j0 + j, ny) * R_NR; };
-
-  // ---- phase A: stage state, mask and thickness ----------------------
-  for (int q = tid; q < NS; q += NT) {
-    int ti = q % W - HALO, tj = q / W - HALO;
-    int gi = wrapi(i0 + ti, nx), gj = wrapi(j0 + tj, ny);
-    size_t k = (size_t)gi + (size_t)nx * gj;
-    uint8_t m = p.mc[k];
-    T e = p.e0[k], he = p.He[k];
-    sM[q] = m;
-    sU[q] = p.u0[k];
-    sV[q] = p.v0[k];
-    sE[q] = e;
-    // computeD: D = eta + H on ocean eta (FULLY_NONLINEAR, land keeps 1),
-    // else the eta-grid depth
-    sD[q] = nl ? ((m & 8) ? e + he : T(1)) : he;
-  }
-  __syncthreads();
-
-  auto oH = [&](int q) { return sM[q] & 1; };
-  auto oU = [&](int q) { return (sM[q] >> 1) & 1; };
-  auto oV = [&](int q) { return (sM[q] >> 2) & 1; };
-  auto oE = [&](int q) { return (sM[q] >> 3) & 1; };
-  auto Du_at = [&](int q) {  // eta2u_noland of D
-    int a = oE(q), b = oE(q - 1);
-    return (T(a) * sD[q] + T(b) * sD[q - 1]) * recip_cnt<T>(a + b);
-  };
-  auto Dv_at = [&](int q) {
-    int a = oE(q), b = oE(q - W);
-    return (T(a) * sD[q] + T(b) * sD[q - W]) * recip_cnt<T>(a + b);
-  };
-  auto Dh_at = [&](int q) {  // eta2H_noland: (i,j),(i-1,j-1),(i-1,j),(i,j-1)
-    int a = oE(q), b = oE(q - W - 1), c = oE(q - 1), d = oE(q - W);
-    return (T(a) * sD[q] + T(b) * sD[q - W - 1] + T(c) * sD[q - 1] + T(d) * sD[q - W]) * recip_cnt<T>(a + b + c + d);
-  };
-  auto inner = [&](int ti, int tj, int lo, int hi_) {
-    return ti >= -HALO + lo && ti < TX + HALO - hi_ && tj >= -HALO + lo && tj < TY + HALO - hi_;
-  };
-
-  // P tensor of the Laplacian-type stress at eta (pll) and H (plt) points for
-  // the velocity pair (a, b) = (u-like, v-like), weights on (weighted) or 1
-  auto p_tensor = [&](const T *a, const T *b, T Ah, bool weighted, T *outL, T *outT) {
-    for (int q = tid; q < NS; q += NT) {
-      int ti = q % W - HALO, tj = q / W - HALO;
-      T pl = T(0), pt = T(0);
-      if (ti < TX + HALO - 1 && tj < TY + HALO - 1 && oE(q)) {  // needs (i+1, j), (i, j+1)
-        const T *r = row(tj);
-        int ov = oV(q), ovp = oV(q + W);
-        T tE = r[R_TE] * recip_cnt<T>(ov + ovp);  // counts 0..2: exactly the division
-        T c0 = Ah * r[R_PC0];
-        T c1 = Ah * (p.q1 + T(ovp) * tE);
-        T c2 = Ah * (-p.q1 + T(ov) * tE);
-        pl = (weighted ? sD[q] : T(1)) * (c0 * (a[q + 1] - a[q]) + c1 * b[q + W] + c2 * b[q]);
-      }
-      if (ti > -HALO && tj > -HALO && oH(q)) {  // needs (i-1, j), (i, j-1)
-        const T *r = row(tj);
-        int ou = oU(q), oum = oU(q - W);
-        T tH = r[R_TH] * recip_cnt<T>(ou + oum);
-        T c0 = Ah * r[R_HC0];
-        T c1 = -Ah * (p.q1 + T(ou) * tH);
-        T c2 = -Ah * (-p.q1 + T(oum) * tH);
-        pt = (weighted ? Dh_at(q) : T(1)) * (c0 * (b[q] - b[q - 1]) + c1 * a[q] + c2 * a[q - W]);
-      }
-      outL[q] = pl;
-      outT[q] = pt;
-    }
-  };
-  // divergence of P onto u and v points (compute_uv); unit thickness or D
-  auto lat_u = [&](int q, int tj, bool weighted) {
-    const T *r = row(tj);
-    int o = oH(q) + oH(q + W);
-    T t2 = T(2) * r[R_TU] * recip_cnt<T>(o);
-    T m0 = -r[R_RU_DL], m1 = -(p.q1 - t2), m2 = p.q1 + t2;
-    T s = m0 * (sPLL[q] - sPLL[q - 1]) + m1 * sPLT[q + W] + m2 * sPLT[q];
-    return weighted ? s / Du_at(q) : s;
-  };
-  auto lat_v = [&](int q, int tj, bool weighted) {
-    const T *r = row(tj);
-    int o = oE(q) + oE(q - W);
-    T t2 = T(2) * r[R_TV] * recip_cnt<T>(o);
-    T m0 = -r[R_RV_DL], m1 = p.q1 - t2, m2 = -(p.q1 + t2);
-    T s = m0 * (sPLT[q + 1] - sPLT[q]) + m1 * sPLL[q] + m2 * sPLL[q - W];
-    return weighted ? s / Dv_at(q) : s;
-  };
-
-  if (p.mix == 2) {
-    // biharmonic extension: first pass with unit thickness and Ah = 1
-    p_tensor(sU, sV, T(1), false, sPLL, sPLT);
-    __syncthreads();
-    for (int q = tid; q < NS; q += NT) {
-      int ti = q % W - HALO, tj = q / W - HALO;
-      bool ok = inner(ti, tj, 1, 1);
-      sLU[q] = (ok && oU(q)) ? lat_u(q, tj, false) : T(0);
-      sLV[q] = (ok && oV(q)) ? lat_v(q, tj, false) : T(0);
-    }
-    __syncthreads();
-  }
-
-  // ---- phase B: mass fluxes, PV, Bernoulli, P tensor -------------------
-  for (int q = tid; q < NS; q += NT) {
-    int ti = q % W - HALO, tj = q / W - HALO;
-    bool lo_ok = ti > -HALO && tj > -HALO;
-    bool hi_ok = ti < TX + HALO - 1 && tj < TY + HALO - 1;
-    sMU[q] = (ti > -HALO && oU(q)) ? Du_at(q) * sU[q] : T(0);
-    sMV[q] = (tj > -HALO && oV(q)) ? Dv_at(q) * sV[q] : T(0);
-    T pot = T(0);
-    if (lo_ok && p.mode != SWM_MODE_NONE) {
-      const T *r = row(tj);
-      T zeta = T(0);
-      if (nl) {
-        T bc = oH(q) ? T(1) : p.lbc;
-        T dvdx = (oV(q - 1) + oV(q) == 0) ? T(0) : bc * r[R_RH_DL] * (sV[q] - sV[q - 1]);
-        T dudy = (oU(q) + oU(q - W) == 0) ? T(0) : bc * p.q1 * (r[R_CU] * sU[q] - row(tj - 1)[R_CU] * sU[q - W]);
-        zeta = dvdx - dudy * r[R_INV_CH];
-      }
-      T pD = Dh_at(q);
-      pD = pD > p.eps ? pD : p.eps;
-      pot = (r[R_FH] + zeta) / pD;
-    }
-    sPOT[q] = pot;
-    T b = T(0);
-    if (hi_ok && oE(q) && p.mode != SWM_MODE_NONE) {
-      b = p.G * sE[q];
-      if (nl) {
-        T a = T(0.5) * (sU[q + 1] * sU[q + 1]) + T(0.5) * (sU[q] * sU[q]);
-        T c = T(0.5) * (sV[q + W] * sV[q + W]) + T(0.5) * (sV[q] * sV[q]);
-        b = (a + c) * T(0.5) + b;
-      }
-    }
-    sB[q] = b;
-  }
-  if (p.mix == 1) p_tensor(sU, sV, p.Ah, true, sPLL, sPLT);
-  if (p.mix == 2) {
-    __syncthreads();  // lat_u/lat_v of the first pass read sPLL/sPLT
-    p_tensor(sLU, sLV, -p.bih, true, sPLL, sPLT);
-  }
-  __syncthreads();
-
-  // ---- phase C: tendencies and Adams-Bashforth update (interior) ------
-  for (int q0 = tid; q0 < TX * TY; q0 += NT) {
-    int ti = q0 % TX, tj = q0 / TX;
-    int gi = i0 + ti, gj = j0 + tj;
-    if (gi >= nx || gj >= ny) continue;
-    size_t k = (size_t)gi + (size_t)nx * gj;
-    int q = S(ti, tj);
-    const T *r = row(tj);
-    T ge = T(0), gu = T(0), gv = T(0);
-    if (oE(q)) {
-      T cvp = row(tj + 1)[R_CV], cv = r[R_CV];
-      ge = -(sMU[q + 1] - sMU[q]) * r[R_RE_DL] - (sMV[q + W] * cvp - sMV[q] * cv) * r[R_RE_DT];
-      if (p.has_F) ge = ge + p.Fe[k];
-    }
-    if (oU(q)) {
-      T pv = T(0.5) * sPOT[q + W] + T(0.5) * sPOT[q];
-      T mv = T(0.25) * sMV[q + W] + T(0.25) * sMV[q - 1] + T(0.25) * sMV[q - 1 + W] + T(0.25) * sMV[q];
-      T g = pv * mv - (sB[q] - sB[q - 1]) * r[R_RU_DL];
-      if (p.qbf) {
-        T vb = T(0.25) * sV[q + W] + T(0.25) * sV[q - 1] + T(0.25) * sV[q - 1 + W] + T(0.25) * sV[q];
-        T gs = p.gsq_uniform ? p.gsq_s[0] : p.gsq[0][k];
-        T f = gs * sqrt(sU[q] * sU[q] + vb * vb) * sU[q];
-        if (p.barotropic) f = f / p.Hu[k];
-        g = g - f;
-      }
-      if (p.mix) g = g + lat_u(q, tj, true);
-      if (p.has_F) g = g + p.Fx[k];
-      if (p.wind_x) g = g + p.ts_rho * (p.wind_rows ? p.wx[gj] : p.wx[k]) / (nl ? Du_at(q) : T(1));
-      gu = g;
-    }
-    if (oV(q)) {
-      T pv = T(0.5) * sPOT[q + 1] + T(0.5) * sPOT[q];
-      T mu = T(0.25) * sMU[q + 1] + T(0.25) * sMU[q - W] + T(0.25) * sMU[q] + T(0.25) * sMU[q + 1 - W];
-      T g = -pv * mu - (sB[q] - sB[q - W]) * p.q1;
-      if (p.qbf) {
-        T ub = T(0.25) * sU[q + 1] + T(0.25) * sU[q - W] + T(0.25) * sU[q] + T(0.25) * sU[q + 1 - W];
-        T gs = p.gsq_uniform ? p.gsq_s[1] : p.gsq[1][k];
-        T f = gs * sqrt(sV[q] * sV[q] + ub * ub) * sV[q];
-        if (p.barotropic) f = f / p.Hv[k];
-        g = g - f;
-      }
-      if (p.mix) g = g + lat_v(q, tj, true);
-      if (p.has_F) g = g + p.Fy[k];
-      if (p.wind_y) g = g + p.ts_rho * (p.wind_rows ? p.wy[gj] : p.wy[k]) / (nl ? Dv_at(q) : T(1));
-      gv = g;
-    }
-    p.Ge3[k] = ge;
-    p.Gu3[k] = gu;
-    p.Gv3[k] = gv;
-    T ie = p.impl_uniform ? p.impl_s[2] : p.impl[2][k];
-    T iu = p.impl_uniform ? p.impl_s[0] : p.impl[0][k];
-    T iv = p.impl_uniform ? p.impl_s[1] : p.impl[1][k];
-    T ince = p.dt * (p.ab0 * p.Ge1[k] + p.ab1 * p.Ge2[k] + p.ab2 * ge);
-    T incu = p.dt * (p.ab0 * p.Gu1[k] + p.ab1 * p.Gu2[k] + p.ab2 * gu);
-    T incv = p.dt * (p.ab0 * p.Gv1[k] + p.ab1 * p.Gv2[k] + p.ab2 * gv);
-    T lim = p.minD - p.He[k];
-    T e = (sE[q] + ince) / ie;
-    if (nl && e < lim) e = lim;
-    p.e1[k] = e;
-    p.u1[k] = (sU[q] + incu) / iu;
-    p.v1[k] = (sV[q] + incv) / iv;
-  }
-}
 
 // FP64 <-> FP32 hi/lo conversions
 __global__ void k_split(const double *src, float *hi, float *lo, size_t n) {
@@ -327,6 +61,7 @@ struct FusedState {
   bool lin_mean = false, dyn_F = false;
   void *Fc[3] = {};
   double *ms_zeta = nullptr, *ms_ex = nullptr;
+  Scratch64 s64;  // FP64 path
 };
 
 namespace swm {
@@ -394,29 +129,15 @@ int fused_prepare(swm_gpu_ctx *c) {
   FTRY(dmalloc((void **)&f->mc, n));
   SWM_CK(cudaMemcpy(f->mc, mc.data(), n, cudaMemcpyHostToDevice));
   // per-row metric factors, from the FP64 grid
-  std::vector<double> rows((size_t)ny * R_NR);
-  double A = cf.A, dL = g.dLambda, dT = g.dTheta;
-  for (int j = 0; j < ny; j++) {
-    double *r = &rows[(size_t)j * R_NR];
-    double cE = g.cosl[GE][j], cV = g.cosl[GV][j], cU = g.cosl[GU][j], cH = g.cosl[GH][j];
-    r[R_CE] = cE;
-    r[R_CV] = cV;
-    r[R_CU] = cU;
-    r[R_FH] = g.f[GH][j];
-    r[R_RE_DL] = 1. / (A * cE * dL);
-    r[R_RE_DT] = 1. / (A * cE * dT);
-    r[R_RU_DL] = 1. / (A * cU * dL);
-    r[R_RV_DL] = 1. / (A * cV * dL);
-    r[R_RH_DL] = 1. / (A * cH * dL);
-    r[R_INV_CH] = 1. / cH;
-    r[R_PC0] = -1. / (dL * A * cE);
-    r[R_HC0] = -1. / (dL * A * cH);
-    r[R_TE] = g.tanl[GE][j] / A;
-    r[R_TH] = g.tanl[GH][j] / A;
-    r[R_TU] = g.tanl[GU][j] / A;
-    r[R_TV] = g.tanl[GV][j] / A;
+  if (!f32) {
+    const std::vector<double> rows = fused64_rows(c);
+    FTRY(upload_t(c, false, rows.data(), rows.size(), &f->rows));
+    const int mix = cf.lateral_mixing ? (cf.mixing_kind == SWM_MIX_BIHARMONIC ? 2 : 1) : 0;
+    Scratch64 &s = f->s64;
+    double **bufs[] = {&s.mu, &s.mv, &s.pot, &s.B, &s.rdu, &s.rdv, &s.pl, &s.pt, &s.dh, &s.lu, &s.lv};
+    const int nb = mix == 2 ? 11 : (mix == 1 ? 8 : 6);
+    for (int q = 0; q < nb; q++) FTRY(dmalloc((void **)bufs[q], n * 8));
   }
-  FTRY(upload_t(c, f32, rows.data(), rows.size(), &f->rows));
   // depths (after computeD at itt = 0)
   std::vector<double> tmp;
   download(c, c->d_H[GE], tmp);
@@ -569,13 +290,15 @@ int fused_sync_state(swm_gpu_ctx *c) {
   return SWM_GPU_OK;
 }
 
-template <typename T>
-static void fill_common(swm_gpu_ctx *c, FP<T> &p, int64_t itt) {
+// parameter block of the FP64 step kernels
+static void make_p64(swm_gpu_ctx *c, int64_t itt, P64 &p) {
   const swm_gpu_config &cf = c->cfg;
-  FusedState *f = c->fused;
+  const FusedState *f = c->fused;
+  memset(&p, 0, sizeof(p));
   p.nx = c->nx;
   p.ny = c->ny;
-  p.mode = cf.mode;
+  p.nl = cf.mode == SWM_MODE_NONLINEAR;
+  p.has_mode = cf.mode != SWM_MODE_NONE;
   p.mix = cf.lateral_mixing ? (cf.mixing_kind == SWM_MIX_BIHARMONIC ? 2 : 1) : 0;
   p.qbf = cf.quadratic_friction;
   p.barotropic = cf.barotropic;
@@ -585,48 +308,41 @@ static void fill_common(swm_gpu_ctx *c, FP<T> &p, int64_t itt) {
   p.wind_x = f->wind_x;
   p.wind_y = f->wind_y;
   p.wind_rows = f->wind_rows;
-  int tstep = (int)(itt < 3 ? itt : 3);
-  p.tstep = tstep;
-  double chi = cf.ab_chi;
-  double tab[4][3] = {{0, 0, 0}, {1., 0, 0}, {-0.5 - chi, 1.5 + chi, 0}, {5. / 12., -16. / 12., 23. / 12.}};
-  p.ab0 = (T)tab[tstep][0];
-  p.ab1 = (T)tab[tstep][1];
-  p.ab2 = (T)tab[tstep][2];
-  p.dt = (T)cf.dt;
+  const int tstep = (int)(itt < 3 ? itt : 3);
+  const double chi = cf.ab_chi;
+  const double tab[4][3] = {{0, 0, 0}, {1., 0, 0}, {-0.5 - chi, 1.5 + chi, 0}, {5. / 12., -16. / 12., 23. / 12.}};
+  p.ab0 = cf.dt * tab[tstep][0];
+  p.ab1 = cf.dt * tab[tstep][1];
+  p.ab2 = cf.dt * tab[tstep][2];
   // without a linearisation define EDens stays 0: no pressure gradient
   // (swm_nonlinear_timestep_module.f90:291-305)
-  p.G = cf.mode == SWM_MODE_NONE ? (T)0 : (T)cf.G;
-  p.minD = (T)cf.minD;
-  p.lbc = (T)cf.lbc;
-  p.q1 = (T)(1. / (cf.A * c->hg.dTheta));
-  p.ts_rho = (T)(cf.tau_scale / cf.RHO0);
-  p.Ah = (T)cf.Ah;
-  p.bih = (T)cf.bih;
-  p.eps = sizeof(T) == 8 ? (T)2.220446049250313e-16 : (T)1.1920929e-07;
-  for (int q = 0; q < 3; q++) p.impl_s[q] = (T)f->impl_s[q];
-  for (int q = 0; q < 2; q++) p.gsq_s[q] = (T)f->gsq_s[q];
+  p.G = cf.mode == SWM_MODE_NONE ? 0. : cf.G;
+  p.minD = cf.minD;
+  p.lbc = cf.lbc;
+  p.q1 = 1. / (cf.A * c->hg.dTheta);
+  p.ts_rho = cf.tau_scale / cf.RHO0;
+  for (int q = 0; q < 3; q++) p.dp_s[q] = (f->impl_s[q] - 1.) / f->impl_s[q];
+  for (int q = 0; q < 2; q++) p.gsq_s[q] = f->gsq_s[q];
   p.mc = f->mc;
-  p.He = (const T *)f->He;
-  p.rows = (const T *)f->rows;
-  p.Hu = (const T *)f->Hu;
-  p.Hv = (const T *)f->Hv;
-  for (int q = 0; q < 3; q++) p.impl[q] = (const T *)f->impl[q];
-  for (int q = 0; q < 2; q++) p.gsq[q] = (const T *)f->gsq[q];
-  p.Fx = (const T *)f->F[0];
-  p.Fy = (const T *)f->F[1];
-  p.Fe = (const T *)f->F[2];
-  p.wx = (const T *)f->wx;
-  p.wy = (const T *)f->wy;
+  p.He = (const double *)f->He;
+  p.rows = (const double *)f->rows;
+  p.Hu = (const double *)f->Hu;
+  p.Hv = (const double *)f->Hv;
+  for (int q = 0; q < 3; q++) p.impl[q] = (const double *)f->impl[q];
+  for (int q = 0; q < 2; q++) p.gsq[q] = (const double *)f->gsq[q];
+  p.Fx = (const double *)f->F[0];
+  p.Fy = (const double *)f->F[1];
+  p.Fe = (const double *)f->F[2];
+  p.wx = (const double *)f->wx;
+  p.wy = (const double *)f->wy;
+  const Dev d = c->dev();
+  p.u0 = d.u0; p.v0 = d.v0; p.e0 = d.eta0;
+  p.u1 = d.u1; p.v1 = d.v1; p.e1 = d.eta1;
+  p.Gu1 = d.Gu[0]; p.Gu2 = d.Gu[1]; p.Gu3 = d.Gu[2];
+  p.Gv1 = d.Gv[0]; p.Gv2 = d.Gv[1]; p.Gv3 = d.Gv[2];
+  p.Ge1 = d.Ge[0]; p.Ge2 = d.Ge[1]; p.Ge3 = d.Ge[2];
+  p.s = f->s64;
 }
-
-template <typename T>
-static void launch_fused(swm_gpu_ctx *c, const FP<T> &p) {
-  dim3 grid((c->nx + TX - 1) / TX, (c->ny + TY - 1) / TY);
-  if (p.mix == 2) k_fused<T, 2><<<grid, NT, 0, c->stream>>>(p);
-  else k_fused<T, 1><<<grid, NT, 0, c->stream>>>(p);
-  c->launches++;
-}
-
 
 // parameter block of the FP32 step kernel for step itt from the context's
 // current level and ring offsets
@@ -1002,16 +718,9 @@ int fused_step(swm_gpu_ctx *c, int64_t itt) {
   FusedState *f = c->fused;
   if (f->dyn_F) FTRY(dyn_forcing(c, itt));
   if (!f->comp) {
-    FP<double> p;
-    memset(&p, 0, sizeof(p));
-    fill_common(c, p, itt);
-    Dev d = c->dev();
-    p.u0 = d.u0; p.v0 = d.v0; p.e0 = d.eta0;
-    p.u1 = d.u1; p.v1 = d.v1; p.e1 = d.eta1;
-    p.Gu1 = d.Gu[0]; p.Gu2 = d.Gu[1]; p.Gu3 = d.Gu[2];
-    p.Gv1 = d.Gv[0]; p.Gv2 = d.Gv[1]; p.Gv3 = d.Gv[2];
-    p.Ge1 = d.Ge[0]; p.Ge2 = d.Ge[1]; p.Ge3 = d.Ge[2];
-    launch_fused<double>(c, p);
+    P64 p;
+    make_p64(c, itt, p);
+    FTRY(fused64_launch(c, p));
   } else {
     FTRY(launch_fp32c(c, itt));
     // the pair state advances here; the host-side advance only rotates the
@@ -1033,6 +742,8 @@ void fused_free(swm_gpu_ctx *c) {
   F(f->mc); F(f->He); F(f->rows); F(f->Hu); F(f->Hv); F(f->wx); F(f->wy); F(f->rows32c); F(f->mask16);
   for (int q = 0; q < 3; q++) { F(f->dp[q]); F(f->Fc[q]); }
   F(f->ms_zeta); F(f->ms_ex);
+  Scratch64 &s = f->s64;
+  F(s.mu); F(s.mv); F(s.pot); F(s.B); F(s.rdu); F(s.rdv); F(s.pl); F(s.pt); F(s.dh); F(s.lu); F(s.lv);
   delete f;
   c->fused = nullptr;
 }
