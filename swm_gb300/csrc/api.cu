@@ -32,12 +32,12 @@ swm::Dev swm_gpu_ctx::dev() const {
   d.RHO0 = cfg.RHO0;
   d.lbc = cfg.lbc;
   d.pdiv = pdiv ? 1 : 0;
-  d.r_dLambda = 1. / hg.dLambda;
-  d.r_dTheta = 1. / hg.dTheta;
-  d.AdT = cfg.A * hg.dTheta;
-  d.r_AdT = 1. / d.AdT;
   d.prow = prow;
-  for (int q = 0; q < 3; q++) d.rimpl[q] = rimpl[q];
+  d.pk = pk;
+  for (int q = 0; q < 3; q++) {
+    d.rimpl[q] = rimpl[q];
+    d.impl_how[q] = pdiv ? impl_how[q] : IMPL_DIVIDE;
+  }
   for (int q = 0; q < 4; q++) {
     d.ocean[q] = d_ocean[q];
     d.cosl[q] = d_cos[q];
@@ -182,8 +182,8 @@ int swm_gpu_destroy(swm_gpu_ctx *c) {
   for (int q = 0; q < 2; q++) { F(c->u[q]); F(c->v[q]); F(c->eta[q]); F(c->gsq[q]); }
   for (int q = 0; q < 3; q++) { F(c->Gu[q]); F(c->Gv[q]); F(c->Ge[q]); F(c->impl[q]); F(c->glin[q]); F(c->F[q]); F(c->Fc[q]); }
   F(c->edens); F(c->pot); F(c->zeta); F(c->mu); F(c->mv); F(c->pll); F(c->plt); F(c->lmu); F(c->lmv);
-  F(c->ones); F(c->latp[0]); F(c->latp[1]); F(c->latuv); F(c->prow); F(c->rimpl[0]); F(c->rimpl[1]);
-  F(c->rimpl[2]); F(c->pdiv_bad); F(c->ubs); F(c->vbs); F(c->zbs); F(c->trc_coeff); F(c->rows_buf); F(c->march_tiles);
+  F(c->latp[0]); F(c->latp[1]); F(c->latuv); F(c->prow); F(c->pk); F(c->rimpl[0]); F(c->rimpl[1]);
+  F(c->rimpl[2]); F(c->pdiv_flags); F(c->ubs); F(c->vbs); F(c->zbs); F(c->trc_coeff); F(c->rows_buf); F(c->march_tiles);
   for (auto &s : c->streams) { F(s.d1); F(s.d2); F(s.rec[0]); F(s.rec[1]); }
   for (auto &t : c->tracers) {
     F(t.CH[0]); F(t.CH[1]); F(t.G[0]); F(t.G[1]); F(t.G[2]); F(t.C); F(t.C0); F(t.gamma); F(t.impl);
@@ -254,8 +254,6 @@ int swm_gpu_domain(swm_gpu_ctx *c, const double *H, const int8_t *Hmiss) {
   }
   if (c->cfg.lateral_mixing && c->cfg.mixing_kind == SWM_MIX_BIHARMONIC) {
     for (int q = 0; q < 4; q++) TRY(dalloc(&c->bh[q], n));
-    TRY(dalloc(&c->ones, n));
-    TRY(plain_fill(c, c->ones, 1.));
   }
   for (int q = 0; q < 3; q++) TRY(plain_fill(c, c->impl[q], 1.));
   c->n0 = 0;
@@ -430,7 +428,9 @@ static int swm_advance_impl(swm_gpu_ctx *c, int64_t itt) {
   c->g0 = (c->g0 + 1) % 3;
   bool plain = c->cfg.path == SWM_PATH_PLAIN_FP64 || itt == 0;
   if (!plain && t64) TRY(fused_sync_state(c));
-  if (plain || t64) {
+  if (c->cfg.path == SWM_PATH_PLAIN_FP64) {
+    TRY(plain_advance(c, itt));
+  } else if (plain || t64) {
     TRY(plain_diagnostics(c, itt));
     TRY(plain_forcing_update(c, itt, 0));
   }
@@ -472,7 +472,10 @@ static bool graph_eligible(const swm_gpu_ctx *c) {
 static int graph_capture(swm_gpu_ctx *c, int64_t itt0) {
   invalidate_graph(c);
   if (c->cfg.path != SWM_PATH_PLAIN_FP64) TRY(fused_prepare(c));  // allocates on first use
-  else TRY(plain_prepare(c));
+  else {
+    TRY(plain_prepare(c));
+    TRY(plain_stress(c));  // the first step's, as after every replay
+  }
   const int n0 = c->n0, g0 = c->g0, phase = (int)(c->advances % GRAPH_STEPS);
   const int64_t l0 = c->launches;
   SWM_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -514,6 +517,7 @@ int swm_gpu_run(swm_gpu_ctx *c, int64_t itt0, int64_t nsteps) {
     if (graphs && itt >= 3 && nsteps - s + 1 >= GRAPH_STEPS) {
       if (!c->graph) TRY(graph_capture(c, itt - 1));
       if (c->advances % GRAPH_STEPS == c->graph_phase) {
+        if (c->cfg.path == SWM_PATH_PLAIN_FP64) TRY(plain_stress(c));
         SWM_CK(cudaGraphLaunch(c->graph, c->stream));
         c->launches += c->graph_launches;
         s += GRAPH_STEPS;
@@ -782,6 +786,7 @@ int swm_gpu_set_field(swm_gpu_ctx *c, int f, const double *in) {
               "swm_gpu_set_field: on the fused paths, set static fields before the first step");
   TRY(h2d(c, p, in, c->n));
   SWM_CK(cudaStreamSynchronize(c->stream));
+  c->stress_ready = false;  // the plain path forms the stress of the next step again
   if (c->cfg.path != SWM_PATH_PLAIN_FP64 && c->stage >= 5 && f <= SWM_F_ETA) TRY(fused_load_state(c));
   if (f == SWM_F_IMPL_U || f == SWM_F_IMPL_V || f == SWM_F_IMPL_ETA) {
     c->pdiv_ready = false;  // the plain path's reciprocals of the damping factors are formed again

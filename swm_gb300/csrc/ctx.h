@@ -91,6 +91,10 @@ struct Tracer {
   int n0 = 0, g0 = 0;
 };
 
+struct PlainRow;    // plain.cu
+struct PlainConst;
+enum { IMPL_DIVIDE, IMPL_SAME, IMPL_FAST };  // per point by the operator; one factor; per point by its reciprocal
+
 // Plain-old-data view of the device state handed to kernels by value.
 struct Dev {
   int nx, ny, mode, qbf, barotropic, lateral_mixing, itt_is_zero;
@@ -98,9 +102,10 @@ struct Dev {
   // the plain path's divisions by fixed divisors (divide.cuh); pdiv 0: the
   // division operator everywhere
   int pdiv;
-  double r_dLambda, r_dTheta, AdT, r_AdT;  // 1/dLambda, 1/dTheta, A dTheta, 1/(A dTheta)
-  const double *prow;                      // PROW_N per row (plain.cu)
-  const double *rimpl[3];                  // 1 / impl_u, _v, _eta
+  int impl_how[3];          // IMPL_*: how u, v, eta are divided by their damping factor
+  const PlainRow *prow;     // per row
+  const PlainConst *pk;     // of the whole grid
+  const double *rimpl[3];   // 1 / impl_u, _v, _eta
   const int8_t *ocean[4];
   const double *cosl[4], *tanl[4], *f[4];
   double *Hg[4];  // H, H_u, H_v, H_eta on the device (H/H_u/H_v overwritten at itt=0 in linear modes)
@@ -144,16 +149,17 @@ struct swm_gpu_ctx {
   double *edens = nullptr, *pot = nullptr, *zeta = nullptr, *mu = nullptr, *mv = nullptr;
   double *pll = nullptr, *plt = nullptr, *lmu = nullptr, *lmv = nullptr;
   double *bh[4] = {};    // biharmonic scratch (first-pass pll, plt, lu, lv)
-  double *ones = nullptr;
   // lateral-mixing coefficients of the plain path per row and mask case
   // (plain.cu k_latmix_tab_*): for up to two values of Ah, and the uv table
   double *latp[2] = {}, latp_ah[2] = {0., 0.}, *latuv = nullptr;
-  // the plain path's fixed divisors and their reciprocals (plain_prepare):
-  // per row A cos_eta, A cos_u dLambda, cos_H and the vorticity factors;
-  // per point 1 / impl_u, _v, _eta; prow_ok: every divisor in div_fast's range
-  double *prow = nullptr, *rimpl[3] = {};
-  int *pdiv_bad = nullptr;
+  // the plain path's fixed divisors (plain_prepare)
+  swm::PlainRow *prow = nullptr;
+  swm::PlainConst *pk = nullptr;
+  double *rimpl[3] = {};
+  unsigned *pdiv_flags = nullptr;
+  int impl_how[3] = {};
   bool pdiv = false, pdiv_ready = false;
+  bool stress_ready = false;  // pll, plt (biharmonic: bh[0], bh[1]) are those of the current state (plain path)
   double *impl[3] = {}, *gsq[2] = {}, *glin[3] = {};
   double *F[3] = {}, *Fc[3] = {};
   double *ubs = nullptr, *vbs = nullptr, *zbs = nullptr;
@@ -194,6 +200,8 @@ void host_damping_finish(swm_gpu_ctx *c);
 // plain.cu
 int plain_diagnostics(swm_gpu_ctx *c, int64_t itt);
 int plain_step(swm_gpu_ctx *c, int64_t itt);
+int plain_advance(swm_gpu_ctx *c, int64_t itt);   // diagnostics, forcing, the next step's stress
+int plain_stress(swm_gpu_ctx *c);                 // the stress, where the state was set since the advance
 int plain_prepare(swm_gpu_ctx *c);                // tables the plain step reads (before a capture)
 int plain_forcing_update(swm_gpu_ctx *c, int64_t itt, int constant_part);
 int plain_fill(swm_gpu_ctx *c, double *p, double value);

@@ -97,10 +97,13 @@ __device__ __forceinline__ FixedDiv fixed_div(double b) {
 
 // a / b, the division operator's quotient bit for bit
 __device__ __forceinline__ double div_fixed(double a, const FixedDiv &d) {
-  if (div_rn_range(a) && d.cls != 2) {
-    double q = div2(a, d.yh, d.yl);
-    if (d.cls) q = __fma_rn(__fma_rn(-q, d.b, a), d.yh, q);
-    return q;
+  if (d.cls != 2) {
+    if (div_rn_range(a)) {
+      double q = div2(a, d.yh, d.yl);
+      if (d.cls) q = __fma_rn(__fma_rn(-q, d.b, a), d.yh, q);
+      return q;
+    }
+    if ((__double_as_longlong(a) << 1) == 0) return __dmul_rn(a, d.yh);  // the zero of the quotient's sign
   }
   return __ddiv_rn(a, d.b);
 }

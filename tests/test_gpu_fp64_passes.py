@@ -1,0 +1,99 @@
+"""The FP64 step kernels against the FP64 oracle at the edges of their blocks
+(32 x 8 points), with every term that has its own branch: mixing, drag,
+damping factors that are one, uniform or vary, wind on either component, land.
+plain_fp64 bit for bit, fused_fp64 to 1e-11 relative L2 after 40 steps (its
+stated tolerance), and a state set between two steps taken up by the next.
+"""
+import numpy as np
+import pytest
+
+from harness import run_case, rel_l2
+from oracle import OracleBackend
+from swm_gb300.host import synthetic
+from swm_gb300.model import GpuModel
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 40
+SIZES = [(30, 6), (31, 7), (32, 8), (63, 15), (64, 17), (97, 23)]   # cells: one point more each way
+
+
+def damping(term, value, varying):
+    return dict(term=term, type=1 if varying else 0, value=value, sl_length=0.02, sl_cutoff=15.0, loc=15,
+                file_data=None)
+
+
+def make(shape, physics):
+    if physics == 'linear':
+        return synthetic.linear_rg(*shape, nsteps=STEPS)
+    case = synthetic.double_gyre(shape, biharmonic=physics == 'biharmonic', nsteps=STEPS)
+    rng = np.random.default_rng(shape[0])
+    H = case['H']
+    case['ic'] = {f: 0.1 * rng.standard_normal(H.shape) for f in ('u', 'v', 'eta')}
+    if physics == 'drag':
+        case['config'].update(quadratic_friction=1)
+        case['damping'] = [damping(0, 1e-5, True), damping(1, 1e-6, False), damping(3, 2e-6, False),
+                           damping(4, 2e-6, False)]
+    if physics == 'winds':   # a second, meridional stress, scaled
+        case['config'].update(lateral_mixing=0, tau_scale=0.7)
+        case['streams'].append(dict(case['streams'][0], comp=1))
+        case['damping'] = [damping(2, 1e-6, True)]
+    return case
+
+
+@pytest.mark.parametrize('path', ['plain_fp64', 'fused_fp64'])
+@pytest.mark.parametrize('physics', ['linear', 'laplacian', 'biharmonic', 'drag', 'winds'])
+def test_block_edges(path, physics):
+    for shape in SIZES:
+        case = make(shape, physics)
+        o, g = OracleBackend(), GpuModel(path)
+        run_case(case, o, nsteps=STEPS, with_diag=False)
+        run_case(case, g, nsteps=STEPS, with_diag=False)
+        for f in ('u', 'v', 'eta'):
+            a, b = g.field(f), o.field(f)
+            if path == 'plain_fp64':
+                assert np.array_equal(a, b), (shape, f)
+            else:
+                err = rel_l2(a, b, o.ocean(f).astype(bool))
+                assert err <= 1e-11, (shape, f, err)
+        g.close()
+
+
+@pytest.mark.parametrize('physics', ['laplacian', 'biharmonic'])
+def test_state_set_between_steps(physics):
+    """plain_fp64 keeps the stress of the advanced state for the next step:
+    u and v set in between are what that step mixes, in single steps and in
+    replayed ones."""
+    case = make((45, 37), physics)
+    rng = np.random.default_rng(5)
+    new = {f: 0.1 * rng.standard_normal(case['H'].shape) for f in ('u', 'v')}
+    runs = []
+    for replay in (True, False):
+        g = GpuModel('plain_fp64')
+        run_case(case, g, nsteps=8, with_diag=False)
+        if replay:
+            g.run(8, 24)
+        else:
+            for itt in range(9, 33):
+                g.step(itt)
+                g.advance(itt)
+        for f, x in new.items():
+            g.set_field(f, x * g.ocean(f))
+        if replay:
+            g.run(32, 24)
+        else:
+            for itt in range(33, 57):
+                g.step(itt)
+                if itt == 33:
+                    mixed = g.field('latmix_u')
+                g.advance(itt)
+        runs.append([g.field(f) for f in ('u', 'v', 'eta')])
+        g.close()
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+    # the mixing of step 33 is that of the new state, not of the advanced one
+    h = GpuModel('plain_fp64')
+    run_case(dict(case, ic={**new, 'eta': case['ic']['eta']}), h, nsteps=1, with_diag=False)
+    scale = np.abs(h.field('latmix_u')).max()
+    assert np.abs(mixed - h.field('latmix_u')).max() < 0.2 * scale
+    h.close()
