@@ -177,9 +177,9 @@ int swm_gpu_step(swm_gpu_ctx *ctx, int64_t itt);
    TRC_advance (tracer_module.f90:133-146) */
 int swm_gpu_advance(swm_gpu_ctx *ctx, int64_t itt);
 /* nsteps iterations of step+advance for itt = itt0+1 .. itt0+nsteps with no
-   time-dependent file forcing in between.  From itt = 3 on, without tracers
-   or oscillating forcing, blocks of six steps replay one captured CUDA graph
-   (bit-identical to single steps) */
+   time-dependent file forcing in between.  From itt = 3 on, without
+   oscillating forcing or FP64 tracers on the fused FP64 path, blocks of six
+   steps replay one captured CUDA graph (bit-identical to single steps) */
 int swm_gpu_run(swm_gpu_ctx *ctx, int64_t itt0, int64_t nsteps);
 
 /* nsteps monitored steps (itt0+1 .. itt0+nsteps) issued without a host wait

@@ -126,7 +126,7 @@ static int d2h(swm_gpu_ctx *c, double *dst, const double *src, size_t count) {
   return SWM_GPU_OK;
 }
 
-static void invalidate_graph(swm_gpu_ctx *c) {
+void swm::invalidate_graph(swm_gpu_ctx *c) {
   if (c->graph) {
     cudaGraphExecDestroy(c->graph);
     c->graph = nullptr;
@@ -454,14 +454,15 @@ int swm_gpu_advance(swm_gpu_ctx *c, int64_t itt) {
   return swm_advance_impl(c, itt);
 }
 
-// From itt = 3 on the Adams-Bashforth weights are fixed, and without tracers
-// or oscillating forcing no kernel argument depends on itt; the pointers
-// cycle with the two time levels and the three increment slots, so a block of
-// six steps is captured once and replayed as a CUDA graph.
+// From itt = 3 on the Adams-Bashforth weights are fixed, and without
+// oscillating forcing no kernel argument depends on itt; the pointers (a
+// tracer's too) cycle with the two time levels and the three increment slots,
+// so a block of six steps is captured once and replayed as a CUDA graph.
 constexpr int GRAPH_STEPS = 6;
 
 static bool graph_eligible(const swm_gpu_ctx *c) {
-  if (!c->tracers.empty() && !trc32_active(c)) return false;
+  // FP64 tracers on a fused path: their steps stay single launches
+  if (!c->tracers.empty() && !trc32_active(c) && c->cfg.path != SWM_PATH_PLAIN_FP64) return false;
   for (const Stream &s : c->streams)
     if (s.type == SWM_FRC_OSC) return false;
   return true;

@@ -236,6 +236,7 @@ void integrals_free(swm_gpu_ctx *c);
 // sor.cu
 void sor_free(swm_gpu_ctx *c);
 // api.cu
+void invalidate_graph(swm_gpu_ctx *c);  // the captured steps no longer hold
 int async_record(swm_gpu_ctx *c, int64_t *ticket);  // ticket for the work queued so far
 // diag.cu
 int device_streamfunction(swm_gpu_ctx *c);
