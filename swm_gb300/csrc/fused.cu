@@ -271,6 +271,44 @@ int fused_load_state(swm_gpu_ctx *c) {
   return SWM_GPU_OK;
 }
 
+// one field (SWM_F_U, _V, _ETA) of the FP64 buffers -> the pair state's
+// current level, for a state the host set; the increments stay
+int fused_load_field(swm_gpu_ctx *c, int field) {
+  FusedState *f = c->fused;
+  if (!f || !f->ready || !f->comp) return SWM_GPU_OK;
+  const int a = f->n0;
+  const unsigned nb = (unsigned)((c->n + 255) / 256);
+  if (field == SWM_F_U) k_split<<<nb, 256, 0, c->stream>>>(c->u[c->n0], f->uh[a], f->ul[a], c->n);
+  else if (field == SWM_F_V) k_split<<<nb, 256, 0, c->stream>>>(c->v[c->n0], f->vh[a], f->vl[a], c->n);
+  else k_split<<<nb, 256, 0, c->stream>>>(c->eta[c->n0], f->eh[a], f->el[a], c->n);
+  c->launches++;
+  SWM_CK(cudaGetLastError());
+  return SWM_GPU_OK;
+}
+
+// one field of the pair state, or its newest increment, -> the FP64 buffer
+// that swm_gpu_get_field reads (other fields need none)
+int fused_sync_field(swm_gpu_ctx *c, int field) {
+  FusedState *f = c->fused;
+  if (!f || !f->ready || !f->comp) return SWM_GPU_OK;
+  const int a = f->n0, g = (f->g0 + 1) % 3, cg = (c->g0 + 1) % 3;
+  const float *hi = nullptr, *lo = nullptr;
+  double *dst = nullptr;
+  switch (field) {
+    case SWM_F_U: hi = f->uh[a]; lo = f->ul[a]; dst = c->u[c->n0]; break;
+    case SWM_F_V: hi = f->vh[a]; lo = f->vl[a]; dst = c->v[c->n0]; break;
+    case SWM_F_ETA: hi = f->eh[a]; lo = f->el[a]; dst = c->eta[c->n0]; break;
+    case SWM_F_GU: hi = f->Gu[g]; dst = c->Gu[cg]; break;
+    case SWM_F_GV: hi = f->Gv[g]; dst = c->Gv[cg]; break;
+    case SWM_F_GETA: hi = f->Ge[g]; dst = c->Ge[cg]; break;
+    default: return SWM_GPU_OK;
+  }
+  k_join<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(hi, lo, dst, c->n);
+  c->launches++;
+  SWM_CK(cudaGetLastError());
+  return SWM_GPU_OK;
+}
+
 // FP32 pair state -> FP64 buffers of the current level (host reads, diagnostics)
 int fused_sync_state(swm_gpu_ctx *c) {
   FusedState *f = c->fused;

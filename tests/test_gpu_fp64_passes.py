@@ -99,6 +99,28 @@ def test_state_set_between_steps(physics):
     h.close()
 
 
+def test_state_set_on_the_pair_path():
+    """A field set on fused_fp32c between two steps changes that field alone:
+    the run that follows is fused_fp64's with the same field set, to the path's
+    stated 1e-5 (fields not read back before are not lost).  Both form every
+    diagnostic from the state they step; plain_fp64 keeps those of its last
+    advance, as the reference's arrays do."""
+    case = make((45, 37), 'biharmonic')
+    new = 0.1 * np.random.default_rng(5).standard_normal(case['H'].shape)
+    out = []
+    for path in ('fused_fp64', 'fused_fp32c'):
+        g = GpuModel(path)
+        run_case(case, g, nsteps=20, with_diag=False)
+        g.set_field('u', new * g.ocean('u'))
+        assert np.allclose(g.field('u'), new * g.ocean('u'), rtol=1e-12, atol=0)
+        g.run(20, 20)
+        out.append({f: g.field(f) for f in ('u', 'v', 'eta')} | {'m': {f: g.ocean(f) for f in ('u', 'v', 'eta')}})
+        g.close()
+    for f in ('u', 'v', 'eta'):
+        err = rel_l2(out[1][f], out[0][f], out[0]['m'][f].astype(bool))
+        assert err <= 1e-5, (f, err)
+
+
 @pytest.mark.parametrize('flux', [0, 1])
 @pytest.mark.parametrize('shape', [(31, 7), (40, 24), (65, 33)])
 def test_tracer_steps_replayed(shape, flux):
