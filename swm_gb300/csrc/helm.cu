@@ -42,11 +42,11 @@ __device__ __forceinline__ float sor32_update(float p, float r, float cxw, float
 __device__ __forceinline__ float face32(float a, float b, float rd2) { return (0.5f * (a + b)) * rd2; }
 
 
-// FP64 coefficients formed once: west and south face coefficients and the
-// reciprocal of the diagonal (the sweeps would otherwise be bound by the
+// FP64 coefficients formed once: west and south face coefficients, the
+// diagonal and its reciprocal (the sweeps would otherwise be bound by the
 // FP64 pipe, which forms them and divides at every point of every sweep)
 __global__ void k_h_coeff64(int nx, int ny, const double *__restrict__ h, double rdx2, double rdy2, double lambda,
-                            double *cx, double *cy, double *rcc) {
+                            double *cx, double *cy, double *cc, double *rcc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
   const size_t k = (size_t)i + (size_t)nx * j;
@@ -57,7 +57,8 @@ __global__ void k_h_coeff64(int nx, int ny, const double *__restrict__ h, double
   const double cyn = j < ny - 1 ? (0.5 * (h[k + nx] + hk)) * rdy2 : 0.;
   cx[k] = cxw;
   cy[k] = cys;
-  rcc[k] = 1. / (-(((cxw + cxe) + cys) + cyn) - lambda);
+  cc[k] = -(((cxw + cxe) + cys) + cyn) - lambda;
+  rcc[k] = 1. / cc[k];
 }
 
 // FP64 sweeps run on a colour-split layout: cell (i, j) of colour (i + j) % 2
@@ -98,20 +99,51 @@ __global__ void k_h_split64(int nx, int ny, int W, double *nat, double *s0, doub
 
 // one colour of an FP64 sweep: off = cw w + ce e + cs s + cn n as nested
 // fused multiply-adds, psi += omega ((rhs - off) / diag - psi) as one more
-// (the arithmetic of orc_helmholtz_sor)
-__global__ void k_h_sweep64(int nx, int ny, int W, Split64 s, int col, double omega) {
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (size_t)W * ny || !s.mask[col][q]) return;
-  const int j = (int)(q / W), i = 2 * (int)(q - (size_t)j * W) + ((j + col) & 1);
-  const double *P = s.psi[col ^ 1];
-  const size_t r0 = (size_t)j * W;
-  const double w = i > 0 ? P[r0 + ((i - 1) >> 1)] : 0., e = i < nx - 1 ? P[r0 + ((i + 1) >> 1)] : 0.;
-  const double so = j > 0 ? P[r0 - W + (i >> 1)] : 0., n = j < ny - 1 ? P[r0 + W + (i >> 1)] : 0.;
-  const double off =
-      __fma_rn(s.c[col][0][q], w, __fma_rn(s.c[col][1][q], e, __fma_rn(s.c[col][2][q], so, s.c[col][3][q] * n)));
-  const double gs = (s.rhs[col][q] - off) * s.rcc[col][q];
-  double *x = s.psi[col];
-  x[q] = __fma_rn(omega, gs - x[q], x[q]);
+// (the arithmetic of orc_helmholtz_sor).  8 FP64 operations and 73 B a cell:
+// at 2048^2 a sweep's two colours cannot take less than 67 us in the FP64
+// pipe, nor less than 45 us of HBM.  A thread has the loads of H64_CELLS cells
+// in flight before it looks at any mask; nothing else hides the time of HBM
+// behind the pipe's (90 us a sweep with one cell and its mask first, 72 now).
+constexpr int H64_CELLS = 2, H64_T = 128;
+struct Colour64 {  // one colour's arrays, and the other colour's psi
+  const double *c[4], *rcc, *rhs, *other;
+  double *psi;
+  const uint8_t *mask;
+};
+__global__ void __launch_bounds__(H64_T) k_h_sweep64(int nx, int ny, unsigned W, Colour64 s, int col, double omega) {
+  const unsigned ns = W * (unsigned)ny, q0 = blockIdx.x * (H64_CELLS * H64_T) + threadIdx.x;
+  const double *P = s.other;
+  double *X = s.psi;
+  double cw[H64_CELLS], ce[H64_CELLS], cs[H64_CELLS], cn[H64_CELLS], w[H64_CELLS], e[H64_CELLS], so[H64_CELLS],
+      n[H64_CELLS], b[H64_CELLS], rc[H64_CELLS], x[H64_CELLS];
+  bool wet[H64_CELLS];
+#pragma unroll
+  for (int u = 0; u < H64_CELLS; u++) {
+    const unsigned q = q0 + u * H64_T;
+    wet[u] = false;
+    if (q >= ns) continue;
+    const unsigned j = q / W, c = q - j * W, par = (j + (unsigned)col) & 1u;  // column i = 2 c + par
+    const unsigned i = 2 * c + par;
+    cw[u] = s.c[0][q];
+    ce[u] = s.c[1][q];
+    cs[u] = s.c[2][q];
+    cn[u] = s.c[3][q];
+    b[u] = s.rhs[q];
+    rc[u] = s.rcc[q];
+    x[u] = X[q];
+    w[u] = i > 0 ? P[q - 1 + par] : 0.;
+    e[u] = i + 1 < (unsigned)nx ? P[q + par] : 0.;
+    so[u] = j > 0 ? P[q - W] : 0.;
+    n[u] = j + 1 < (unsigned)ny ? P[q + W] : 0.;
+    wet[u] = s.mask[q] != 0;
+  }
+#pragma unroll
+  for (int u = 0; u < H64_CELLS; u++) {
+    if (!wet[u]) continue;
+    const double off = __fma_rn(cw[u], w[u], __fma_rn(ce[u], e[u], __fma_rn(cs[u], so[u], cn[u] * n[u])));
+    const double gs = (b[u] - off) * rc[u];
+    X[q0 + u * H64_T] = __fma_rn(omega, gs - x[u], x[u]);
+  }
 }
 
 // one colour of an FP32 sweep over the whole grid (the arithmetic of k_h_tbr)
@@ -249,35 +281,79 @@ __global__ void __launch_bounds__(32 * TBR_Y, 2) k_h_tbr(int nx, int ny, const f
   }
 }
 
-// r = rhs - A psi on ocean cells (0 elsewhere) from the FP64 face
-// coefficients, for an FP64 or FP32 iterate; per-block partial sums of r^2
+// out = A psi on ocean cells (0 elsewhere), every product and sum rounded, in
+// the order of orc_helmholtz_apply
+__global__ void k_h_apply(int nx, int ny, const double *__restrict__ cx, const double *__restrict__ cy,
+                          const double *__restrict__ cc, const int8_t *__restrict__ mask,
+                          const double *__restrict__ psi, double *out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= nx || j >= ny) return;
+  const size_t k = (size_t)i + (size_t)nx * j;
+  double a = 0.;
+  if (mask[k]) {
+    const double cxe = i < nx - 1 ? cx[k + 1] : 0., cyn = j < ny - 1 ? cy[k + nx] : 0.;
+    const double w = i > 0 ? psi[k - 1] : 0., e = i < nx - 1 ? psi[k + 1] : 0.;
+    const double s = j > 0 ? psi[k - nx] : 0., nn = j < ny - 1 ? psi[k + nx] : 0.;
+    a = cx[k] * w + cxe * e + cy[k] * s + cyn * nn + cc[k] * psi[k];
+  }
+  out[k] = -(0. - a);
+}
+
+// x in FP64: a normal number's or zero's bits are moved by integer operations
+// (a conversion instruction takes the FP64 pipe's time)
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = (b >> 23) & 255u;
+  if (e - 1u < 254u) return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+  if ((b << 1) == 0) return __hiloint2double((int)b, 0);
+  return (double)x;
+}
+
+// r = rhs - A psi on ocean cells (0 elsewhere; r may be null) for an FP64 or
+// FP32 iterate, and per-block sums of r^2.  FP64-pipe bound: a thread walks
+// RES_ROWS rows of a column, so that a row's values are converted once, the
+// diagonal is read and not added up, and products are fused: 7 FP64
+// operations a cell.  4096^2: 684 us (FP32 iterate) and 554 us (FP64) with 20
+// and 16 operations, 339 and 234 us now; the coefficients, mask, right-hand
+// side and iterate, 33 to 41 B a cell, take about 110 us of HBM.
+constexpr int RES_X = 128, RES_ROWS = 32;
 template <typename T>
-__global__ void k_h_resid_c(int nx, int ny, const double *__restrict__ cx, const double *__restrict__ cy,
-                            double lambda, const int8_t *__restrict__ mask, const T *__restrict__ rhs,
-                            const T *__restrict__ psi, double *r, double *partial) {
-  __shared__ double red[256];
+__global__ void __launch_bounds__(RES_X) k_h_resid(int nx, int ny, const double *__restrict__ cx,
+                                                   const double *__restrict__ cy, const double *__restrict__ cc,
+                                                   const int8_t *__restrict__ mask, const T *__restrict__ rhs,
+                                                   const T *__restrict__ psi, double *r, double *partial) {
+  __shared__ double red[RES_X / 32];
+  const int i = blockIdx.x * RES_X + threadIdx.x, j0 = blockIdx.y * RES_ROWS, j1 = min(j0 + RES_ROWS, ny);
   double acc = 0.;
-  const size_t n = (size_t)nx * ny;
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(k % nx), j = (int)(k / nx);
-    double rr = 0.;
-    if (mask[k]) {
-      const double cxw = cx[k], cxe = i < nx - 1 ? cx[k + 1] : 0., cys = cy[k], cyn = j < ny - 1 ? cy[k + nx] : 0.;
-      const double cc = -(((cxw + cxe) + cys) + cyn) - lambda;
-      const double w = i > 0 ? (double)psi[k - 1] : 0., e = i < nx - 1 ? (double)psi[k + 1] : 0.;
-      const double s = j > 0 ? (double)psi[k - nx] : 0., nn = j < ny - 1 ? (double)psi[k + nx] : 0.;
-      rr = (double)rhs[k] - (cxw * w + cxe * e + cys * s + cyn * nn + cc * (double)psi[k]);
+  if (i < nx) {
+    size_t k = (size_t)i + (size_t)nx * j0;
+    double s = j0 > 0 ? widen(psi[k - nx]) : 0., p = widen(psi[k]), cys = cy[k];
+#pragma unroll 2
+    for (int j = j0; j < j1; j++, k += nx) {
+      const bool top = j == ny - 1;
+      const double n = top ? 0. : widen(psi[k + nx]), cyn = top ? 0. : cy[k + nx];
+      double rr = 0.;
+      if (mask[k]) {
+        const double w = i > 0 ? widen(psi[k - 1]) : 0., e = i < nx - 1 ? widen(psi[k + 1]) : 0.;
+        const double cxe = i < nx - 1 ? cx[k + 1] : 0.;
+        const double off = __fma_rn(cx[k], w, __fma_rn(cxe, e, __fma_rn(cys, s, cyn * n)));
+        rr = widen(rhs[k]) - __fma_rn(cc[k], p, off);
+        acc = __fma_rn(rr, rr, acc);
+      }
+      if (r) r[k] = rr;
+      s = p;
+      p = n;
+      cys = cyn;
     }
-    if (r) r[k] = rr;
-    acc += rr * rr;
   }
-  red[threadIdx.x] = acc;
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = red[0];
+    for (int w = 1; w < RES_X / 32; w++) t += red[w];
+    partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
 __global__ void k_h_sumsq(const double *x, const int8_t *mask, size_t n, double *partial) {
@@ -324,7 +400,7 @@ __global__ void k_h_axpy(double *psi, const float *e32, size_t n, double scale) 
 
 struct swm_helm {
   int device = -1;  // the CUDA device the solver was created on
-  double *cx = nullptr, *cy = nullptr, *rcc = nullptr;  // FP64 coefficients
+  double *cx = nullptr, *cy = nullptr, *cc = nullptr, *rcc = nullptr;  // FP64 coefficients
   swm::Split64 s64 = {};  // the FP64 sweeps' colour-split arrays (first FP64 solve)
   bool has_s64 = false;
   int W = 0;              // cells of a colour-split row
@@ -355,9 +431,13 @@ dim3 sweep_grid(const swm_helm *h, dim3 b) {
 }
 
 void sweep64(swm_helm *h, double omega) {
-  const unsigned g = (unsigned)(((size_t)h->W * h->ny + 255) / 256);
-  for (int colour = 0; colour < 2; colour++)
-    k_h_sweep64<<<g, 256, 0, h->stream>>>(h->nx, h->ny, h->W, h->s64, colour, omega);
+  const unsigned per = H64_CELLS * H64_T, g = (unsigned)(((size_t)h->W * h->ny + per - 1) / per);
+  const Split64 &s = h->s64;
+  for (int colour = 0; colour < 2; colour++) {
+    const Colour64 a = {{s.c[colour][0], s.c[colour][1], s.c[colour][2], s.c[colour][3]}, s.rcc[colour], s.rhs[colour],
+                        s.psi[colour ^ 1], s.psi[colour], s.mask[colour]};
+    k_h_sweep64<<<g, H64_T, 0, h->stream>>>(h->nx, h->ny, h->W, a, colour, omega);
+  }
   h->launches += 2;
 }
 
@@ -425,13 +505,15 @@ void sweeps_tb32(swm_helm *h, float omega, int n) {
   }
 }
 
+// blocks of k_h_resid
+dim3 resid_grid(int nx, int ny) { return dim3((nx + RES_X - 1) / RES_X, (ny + RES_ROWS - 1) / RES_ROWS); }
+
 // ||rhs - A psi||^2 (FP64 accumulation); r written when wanted
 template <typename T>
-int resid2(swm_helm *h, const T *hh, const T *rhs, const T *psi, double *r, double *out) {
-  (void)hh;
-  k_h_resid_c<T><<<HELM_RED, 256, 0, h->stream>>>(h->nx, h->ny, h->cx, h->cy, h->lambda, h->mask, rhs, psi, r,
-                                                  h->partial);
-  k_h_final<<<1, 256, 0, h->stream>>>(h->partial, HELM_RED, h->out);
+int resid2(swm_helm *h, const T *rhs, const T *psi, double *r, double *out) {
+  const dim3 g = resid_grid(h->nx, h->ny);
+  k_h_resid<T><<<g, RES_X, 0, h->stream>>>(h->nx, h->ny, h->cx, h->cy, h->cc, h->mask, rhs, psi, r, h->partial);
+  k_h_final<<<1, 256, 0, h->stream>>>(h->partial, (int)(g.x * g.y), h->out);
   h->launches += 2;
   SWM_CK(cudaGetLastError());
   SWM_CK(cudaMemcpyAsync(h->host, h->out, 8, cudaMemcpyDeviceToHost, h->stream));
@@ -459,7 +541,7 @@ constexpr double STALL = 0.7;
 int inner32(swm_helm *h, float omega, double tol, int max_sweeps, int *sweeps, double *rel) {
   double rn2 = 0.;
   // ||r32||: residual of e = 0
-  HTRY(resid2<float>(h, h->hinv32, h->r32, h->e32, nullptr, &rn2));
+  HTRY(resid2<float>(h, h->r32, h->e32, nullptr, &rn2));
   const double rn = std::sqrt(rn2);
   int s = 0, checks = 0;
   double rr = 1., prev = 1.;
@@ -471,7 +553,7 @@ int inner32(swm_helm *h, float omega, double tol, int max_sweeps, int *sweeps, d
     for (int q = tb; q < blk; q++) sweep32(h, omega, h->blk);
     s += blk;
     double e2 = 0.;
-    HTRY(resid2<float>(h, h->hinv32, h->r32, h->e32, nullptr, &e2));
+    HTRY(resid2<float>(h, h->r32, h->e32, nullptr, &e2));
     rr = rn > 0 ? std::sqrt(e2) / rn : 0.;
     if (rr <= tol || (++checks >= 2 && rr > STALL * prev)) break;
     prev = rr;
@@ -487,7 +569,7 @@ void helm_free(swm_helm *h) {
   cudaFree(h->hinv); cudaFree(h->psi); cudaFree(h->rhs); cudaFree(h->r); cudaFree(h->partial); cudaFree(h->out);
   cudaFreeHost(h->host);
   cudaFree(h->hinv32); cudaFree(h->e32); cudaFree(h->r32); cudaFree(h->mask); cudaFree(h->e32b);
-  cudaFree(h->cx); cudaFree(h->cy); cudaFree(h->rcc);
+  cudaFree(h->cx); cudaFree(h->cy); cudaFree(h->cc); cudaFree(h->rcc);
   for (int col = 0; col < 2; col++) {
     for (int f = 0; f < 4; f++) cudaFree(h->s64.c[col][f]);
     cudaFree(h->s64.rcc[col]); cudaFree(h->s64.rhs[col]); cudaFree(h->s64.psi[col]); cudaFree(h->s64.mask[col]);
@@ -519,16 +601,17 @@ int swm_helm_create(int nx, int ny, double dx, double dy, double lambda, const d
     hinv[k] = 1. / H[k];
     hinv32[k] = (float)hinv[k];
   }
+  const dim3 rg = resid_grid(nx, ny);
   bool ok = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaMalloc((void **)&h->hinv, n * 8) == cudaSuccess && cudaMalloc((void **)&h->psi, n * 8) == cudaSuccess &&
             cudaMalloc((void **)&h->rhs, n * 8) == cudaSuccess && cudaMalloc((void **)&h->r, n * 8) == cudaSuccess &&
-            cudaMalloc((void **)&h->partial, HELM_RED * 8) == cudaSuccess &&
+            cudaMalloc((void **)&h->partial, std::max<size_t>(HELM_RED, (size_t)rg.x * rg.y) * 8) == cudaSuccess &&
             cudaMalloc((void **)&h->out, 8) == cudaSuccess && cudaMallocHost((void **)&h->host, 8) == cudaSuccess &&
             cudaMalloc((void **)&h->hinv32, n * 4) == cudaSuccess && cudaMalloc((void **)&h->e32, n * 4) == cudaSuccess &&
             cudaMalloc((void **)&h->r32, n * 4) == cudaSuccess && cudaMalloc((void **)&h->mask, n) == cudaSuccess &&
             cudaMalloc((void **)&h->e32b, n * 4) == cudaSuccess &&
             cudaMalloc((void **)&h->cx, n * 8) == cudaSuccess && cudaMalloc((void **)&h->cy, n * 8) == cudaSuccess &&
-            cudaMalloc((void **)&h->rcc, n * 8) == cudaSuccess;
+            cudaMalloc((void **)&h->cc, n * 8) == cudaSuccess && cudaMalloc((void **)&h->rcc, n * 8) == cudaSuccess;
   if (!ok) {
     helm_free(h);
     set_error("swm_helm_create: device allocation failed");
@@ -538,7 +621,7 @@ int swm_helm_create(int nx, int ny, double dx, double dy, double lambda, const d
   SWM_CK(cudaMemcpyAsync(h->hinv32, hinv32.data(), n * 4, cudaMemcpyHostToDevice, h->stream));
   SWM_CK(cudaMemcpyAsync(h->mask, ocean, n, cudaMemcpyHostToDevice, h->stream));
   dim3 b(32, 8), g((nx + 31) / 32, (ny + 7) / 8);
-  k_h_coeff64<<<g, b, 0, h->stream>>>(nx, ny, h->hinv, 1. / (dx * dx), 1. / (dy * dy), lambda, h->cx, h->cy, h->rcc);
+  k_h_coeff64<<<g, b, 0, h->stream>>>(nx, ny, h->hinv, 1. / (dx * dx), 1. / (dy * dy), lambda, h->cx, h->cy, h->cc, h->rcc);
   h->launches++;
   SWM_CK(cudaGetLastError());
   SWM_CK(cudaStreamSynchronize(h->stream));
@@ -560,12 +643,12 @@ int swm_helm_apply(swm_helm *h, const double *psi, double *out) {
   SWM_ON_DEVICE(h ? h->device : -1);
   SWM_REQUIRE(h && psi && out, "swm_helm_apply: bad arguments");
   SWM_CK(cudaMemcpyAsync(h->psi, psi, h->n * 8, cudaMemcpyHostToDevice, h->stream));
-  SWM_CK(cudaMemsetAsync(h->rhs, 0, h->n * 8, h->stream));
-  double r2;
-  HTRY(resid2<double>(h, h->hinv, h->rhs, h->psi, h->r, &r2));  // r = 0 - A psi
-  std::vector<double> t(h->n);
-  SWM_CK(cudaMemcpy(t.data(), h->r, h->n * 8, cudaMemcpyDeviceToHost));
-  for (size_t k = 0; k < h->n; k++) out[k] = -t[k];
+  const dim3 b(32, 8), g((h->nx + 31) / 32, (h->ny + 7) / 8);
+  k_h_apply<<<g, b, 0, h->stream>>>(h->nx, h->ny, h->cx, h->cy, h->cc, h->mask, h->psi, h->r);
+  h->launches++;
+  SWM_CK(cudaGetLastError());
+  SWM_CK(cudaMemcpyAsync(out, h->r, h->n * 8, cudaMemcpyDeviceToHost, h->stream));
+  SWM_CK(cudaStreamSynchronize(h->stream));
   return SWM_GPU_OK;
 }
 
@@ -590,7 +673,7 @@ int swm_helm_solve_fp64(swm_helm *h, const double *rhs, double *psi, double omeg
     s += blk;
     split64_field(h, h->psi, h->s64.psi, 1);  // the residual reads the natural layout
     double r2;
-    HTRY(resid2<double>(h, h->hinv, h->rhs, h->psi, nullptr, &r2));
+    HTRY(resid2<double>(h, h->rhs, h->psi, nullptr, &r2));
     rel = bn > 0 ? std::sqrt(r2) / bn : std::sqrt(r2);
     if (rel < rtol) break;
   }
@@ -619,7 +702,7 @@ int swm_helm_solve_mixed(swm_helm *h, const double *rhs, double *psi, double ome
   double rel = 1.;
   for (;;) {
     double r2;
-    HTRY(resid2<double>(h, h->hinv, h->rhs, h->psi, h->r, &r2));
+    HTRY(resid2<double>(h, h->rhs, h->psi, h->r, &r2));
     const double rn = std::sqrt(r2);
     rel = bn > 0 ? rn / bn : rn;
     if (rel < rtol || s >= max_sweeps || rn == 0.) break;
@@ -711,7 +794,7 @@ int swm_helm_autotune(swm_helm *h, const double *rhs, double omega_lo, double om
     sweeps_tb32(h, (float)om, tb);
     for (int s = tb; s < trial_sweeps; s++) sweep32(h, (float)om, h->blk);
     double e2;
-    HTRY(resid2<float>(h, h->hinv32, h->r32, h->e32, nullptr, &e2));
+    HTRY(resid2<float>(h, h->r32, h->e32, nullptr, &e2));
     if (e2 < rbest) { rbest = e2; best = om; }
   }
   if (omega) *omega = best;
