@@ -1,5 +1,5 @@
-// trc32.cu -- passive tracers on the FP32 compensated path, all tracers of a
-// basin in one kernel per step.
+// trc32.cu -- passive tracers on the FP32 compensated path, up to two tracers
+// of a basin per launch.
 //
 // Formulas: TRC_tracer_incr (tracer_module.f90:154-209), TRC_initCoeffs
 // (:291-342, coefficients rebuilt from the masks and per-row metric factors,
@@ -16,13 +16,14 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include "ctx.h"
 #include "fused32.h"
 
 namespace swm {
 
-constexpr int TRC32_MAX = 4;  // tracers per launch (more run in several launches)
+constexpr int TRC32_MAX = 2;  // tracers per launch (more run in several launches)
 enum { RT_RDL, RT_RDT, RT_CV, RT_D8, RT_D10, RT_NR };
 
 struct Tracer32 {
@@ -34,7 +35,7 @@ struct Tracer32 {
 };
 
 struct TrcP {
-  int nx, ny, nl, flux, ntr, pf;
+  int nx, ny, nl, flux, ntr, pf, decay;  // decay: a tracer of the launch has an implicit decay
   float dt, ab0, ab1, ab2;
   const float *u, *v, *eta, *He, *Fe, *rows;
   const uint16_t *mask16;
@@ -50,62 +51,109 @@ __device__ __forceinline__ int wr(int a, int n) { return a < 0 ? a + n : (a >= n
 // 1 / thickness, 0 on dry land (C = CH * rD then takes the 0/0 there as 0)
 __device__ __forceinline__ float rthick(float d) { return d != 0.f ? __frcp_rn(d) : 0.f; }
 
-// face value of CH between L and R (R east/north of L), Lm behind L, Rp beyond R
-__device__ __forceinline__ float face(int flux, float vel, float cLm, float cL, float cR, float cRp, unsigned oLm,
-                                      unsigned oL, unsigned oR, unsigned oRp) {
-  if (flux == 1 && oLm && oL && oR && oRp)
-    return vel >= 0.f ? (5.f * cL + 2.f * cR - cLm) * (1.f / 6.f) : (2.f * cL + 5.f * cR - cRp) * (1.f / 6.f);
-  unsigned den = oL + oR;
-  if (den == 0) return 0.f;
-  return (oL ? cL : 0.f) * (den == 2 ? 0.5f : 1.f) + (oR ? cR : 0.f) * (den == 2 ? 0.5f : 1.f);
-}
-
-// (hi + lo + inc) * (1 - dp) as a new (hi, lo) pair, the two roundings
-// recovered by Fast2Sum (Dekker 1971): exact for s - c (c = s dp, 0 <= dp <
-// 1), and for hi + inc wherever the increment is below the tracer content,
-// which fails only where the content passes through zero
-__device__ __forceinline__ void comp_update(float hi, float lo, float inc, float dp, float &nh, float &nl) {
-  const float s = hi + inc;
-  float e = (inc - (s - hi)) + lo;
-  const float c = s * dp;
-  const float t = s - c;
-  const float e2 = (s - t) - c;
-  e = e + e2 - e * dp;
-  nh = t + e;
-  nl = e - (nh - t);
-}
+// One tracer's values (float) or two tracers' (float2): the arithmetic of two
+// runs in packed FP32x2 instructions, each half rounded as the scalar one, so
+// a tracer's results do not depend on how many share its launch.  Every
+// operation below is explicit, with the products that the compiler fused into
+// the sums of the scalar form fused here: results are that form's bit for bit.
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+template <typename V>
+__device__ __forceinline__ V vb(float s);  // s in every half
+template <>
+__device__ __forceinline__ float vb<float>(float s) { return s; }
+template <>
+__device__ __forceinline__ float2 vb<float2>(float s) { return make_float2(s, s); }
+__device__ __forceinline__ float &half(float &v, int) { return v; }
+__device__ __forceinline__ float &half(float2 &v, int q) { return q ? v.y : v.x; }
+__device__ __forceinline__ float vsel(bool c, float a, float b) { return c ? a : b; }
+__device__ __forceinline__ float2 vsel(bool c, float2 a, float2 b) { return make_float2(c ? a.x : b.x, c ? a.y : b.y); }
 
 constexpr unsigned FULLM = 0xffffffffu;
 constexpr int TRC_ROWS = 16;  // output rows per warp
+__device__ __forceinline__ float vup(float v) { return __shfl_up_sync(FULLM, v, 1); }
+__device__ __forceinline__ float2 vup(float2 v) { return make_float2(vup(v.x), vup(v.y)); }
+__device__ __forceinline__ float vdown(float v, int n) { return __shfl_down_sync(FULLM, v, n); }
+__device__ __forceinline__ float2 vdown(float2 v, int n) { return make_float2(vdown(v.x, n), vdown(v.y, n)); }
+
+// Advective flux of CH through the face between L and R (R east or north of
+// L, Lm behind L, Rp beyond R) for the velocity vel (times the row's cosine at
+// a north face): the third-order upwind-biased value (-1, 5, 2)/6 from the
+// upwind side where all four cells are ocean (FLUX 1), the mask-weighted mean
+// elsewhere.  FAST: all masks are 1.
+template <bool FAST, int FLUX, typename V>
+__device__ __forceinline__ V face_flux(float vel, V cLm, V cL, V cR, V cRp, unsigned open, unsigned oLm, unsigned oL,
+                                       unsigned oR, unsigned oRp) {
+  V f;
+  if (FLUX == 1) {
+    const bool pos = vel >= 0.f;
+    const V kL = vb<V>(pos ? 5.f : 2.f), kR = vb<V>(pos ? 2.f : 5.f);
+    const V t = vsub(vfma(kL, cL, vmul(kR, cR)), vsel(pos, cLm, cRp));
+    f = vmul(vmul(t, vb<V>(1.f / 6.f)), vb<V>(vel));
+    if (FAST) return f;
+  }
+  if (FAST) return vmul(vadd(cL, cR), vb<V>(0.5f * vel));
+  const unsigned den = oL + oR;
+  const V zero = vb<V>(0.f);
+  const V mean = vmul(vadd(vsel(oL, cL, zero), vsel(oR, cR, zero)), vb<V>(den == 2 ? 0.5f * vel : vel));
+  if (FLUX == 1 && (oLm & oL & oR & oRp)) return vsel(open, f, zero);
+  return vsel(open && den, mean, zero);
+}
+
+// (hi + lo + inc) * (1 - dp) as a new (hi, lo) pair, inc = dt x (not rounded
+// by itself), the two roundings recovered by Fast2Sum (Dekker 1971): exact for
+// s - c (c = s dp, 0 <= dp < 1), and for hi + inc wherever the increment is
+// below the tracer content, which fails only where the content passes through
+// zero.  ndp = -dp; decay false: dp is 0, and e2 with it.
+template <typename V>
+__device__ __forceinline__ void comp_update(V hi, V lo, V dt, V x, bool decay, V ndp, V &nh, V &nl) {
+  const V s = vfma(dt, x, hi);
+  V e = vadd(vfma(dt, x, vsub(hi, s)), lo), t = s;
+  if (decay) {
+    t = vfma(s, ndp, s);
+    const V e2 = vfma(s, ndp, vsub(s, t));
+    e = vfma(e, ndp, vadd(e, e2));
+  }
+  nh = vadd(t, e);
+  nl = vsub(e, vsub(nh, t));
+}
 
 // One warp owns a strip of 32 columns (lane = column; 2 halo lanes per side,
-// as the upwind-biased faces reach two cells) and TRC_ROWS output rows; it
-// walks up the strip keeping the last five rows of CH (hi + lo), thickness
-// and masks in registers, and updates row J-2 once row J is in.
+// as the upwind-biased faces reach two cells) and S output rows; it walks up
+// the strip keeping the last rows of CH (hi + lo), thickness and masks in
+// registers, and updates row J-2 once row J is in.
+// Issue-bound: where the whole window of a warp is ocean (a warp vote) a body
+// with every mask test folded away runs, and two tracers share packed
+// instructions.  2049^2, two tracers, upwind-biased: 117 us a step with the mask
+// tests and two scalar tracers, 89 now; 2.83 -> 3.66 TB/s of the 78 B a point.
 // PF 1: each iteration also asks L2 for the input rows two beyond those it
 // loads and for the update inputs of the output row after next, so that a
-// state larger than L2 does not make the warp wait on DRAM (trc_prefetch).
-// Resident blocks per SM asked of the register allocator: one tracer fits 6
-// (80 registers, no spill; 2049^2 step 76.0 us against 83.8 at 4), two
-// tracers 4 (at 5 they spill and run slower), three 4 with the updated row's
-// CH pair reloaded instead of carried (RELOAD; 2049^2 step 169 us against
-// 176 at 3 blocks), four 3.
+// state larger than L2 does not make the warp wait on DRAM (trc_prefetch):
+// lanes 2 f and 2 f + 1 ask for the two ends of field f's row segment.
+// Resident blocks per SM asked of the register allocator: 6 with one tracer,
+// 4 with two.
 template <int NT, int FLUX, int PF>
-__global__ void __launch_bounds__(128, NT == 1 ? 6 : (NT <= 3 ? 4 : 3)) k_trc32(TrcP p, int S, int nstrips) {
-  constexpr bool RELOAD = NT == 3;
+__global__ void __launch_bounds__(128, NT == 1 ? 6 : 4) k_trc32(TrcP p, int S, int nstrips) {
+  using V = typename std::conditional<NT == 2, float2, float>::type;
   constexpr int H = 2, TI = 32 - 2 * H;
   const int lane = threadIdx.x & 31;
   // block b: strip b % nstrips, its four warps four consecutive row groups
   const int nx = p.nx, ny = p.ny;
   const int ry0 = ((blockIdx.x / nstrips) * 4 + (threadIdx.x >> 5)) * S;
   if (ry0 >= ny) return;  // whole warp leaves together
-  const int gx = (blockIdx.x % nstrips) * TI - H + lane;
+  const int gx0 = (blockIdx.x % nstrips) * TI - H, gx = gx0 + lane;
   const int gi = wr(gx, nx);
   const bool store_lane = lane >= H && lane < 32 - H && gx < nx;
 
-  unsigned m[5] = {};
-  float D[5] = {}, rD[5] = {}, u[3] = {}, v[3] = {};
-  float chs[NT][5] = {}, chh[NT][3] = {}, chl[NT][3] = {};
+  unsigned m[4] = {};
+  float D[4] = {}, rD[4] = {}, u[3] = {}, v[3] = {};
+  V chs[4] = {}, chh[3] = {}, chl[3] = {};
   int off[3] = {};
   const float *rr[3] = {};
 
@@ -116,7 +164,8 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : (NT <= 3 ? 4 : 3)) k_trc32(
   // 1-2, C0) one output row ahead
   struct Row {
     unsigned m;
-    float D, u, v, h[NT], l[NT];
+    float D, u, v;
+    V h, l;
     int off;
     const float *rows;
   };
@@ -131,24 +180,124 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : (NT <= 3 ? 4 : 3)) k_trc32(
     r.v = p.v[k];
 #pragma unroll
     for (int q = 0; q < NT; q++) {
-      r.h[q] = p.t[q].ch[k];
-      r.l[q] = p.t[q].cl[k];
+      half(r.h, q) = p.t[q].ch[k];
+      half(r.l, q) = p.t[q].cl[k];
     }
   };
   Row n1, n2;
   load(J, n1);
   load(J + 1, n2);
-  float pg1[NT] = {}, pg2[NT] = {}, pc0[NT] = {};
-  float fyp[NT] = {};  // flux through the north faces of the previous output row
+  V pg1 = {}, pg2 = {}, pc0 = {};
+  V fyp = {};  // flux through the north faces of the previous output row
+
+  // the lane's prefetches: an input field of row J + 4, or an update input of
+  // output row J
+  const char *pfp = nullptr;
+  int pfs = 4;
+  bool pfi = false;
+  if (PF) {
+    const int f = lane >> 1, e = (lane & 1) * 31;
+    const void *b = nullptr;
+    switch (f) {
+      case 0: b = p.mask16; pfs = 2; break;
+      case 1: b = p.He; break;
+      case 2: b = p.nl ? p.eta : nullptr; break;
+      case 3: b = p.u; break;
+      case 4: b = p.v; break;
+      case 5: b = p.t[0].ch; break;
+      case 6: b = p.t[0].cl; break;
+      case 7: b = NT == 2 ? p.t[NT - 1].ch : nullptr; break;
+      case 8: b = NT == 2 ? p.t[NT - 1].cl : nullptr; break;
+      case 9: b = p.t[0].G1; break;
+      case 10: b = p.t[0].G2; break;
+      case 11: b = p.t[0].C0; break;
+      case 12: b = NT == 2 ? p.t[NT - 1].G1 : nullptr; break;
+      case 13: b = NT == 2 ? p.t[NT - 1].G2 : nullptr; break;
+      case 14: b = NT == 2 ? p.t[NT - 1].C0 : nullptr; break;
+      default: break;
+    }
+    pfi = f >= 9;
+    if (b) pfp = static_cast<const char *>(b) + (size_t)(((gx0 + e) % nx + nx) % nx) * pfs;
+  }
+
+  auto body = [&](auto fast_tag) {
+    constexpr bool FAST = decltype(fast_tag)::value;
+    const int o = J - 2;
+    const bool upd = store_lane && o >= ry0 && o < ny;
+    // masks of row o and its neighbours
+    const unsigned mo = m[2];
+    unsigned oE = 1, oEim = 1, oEip = 1, oUip = 1, oV = 1, oVjp = 1, oEjp = 1, oEjm = 1, oEipp = 1, oEjpp = 1;
+    if (!FAST) {
+      oE = (mo >> 3) & 1; oEim = (mo >> 7) & 1; oEip = (mo >> 11) & 1;
+      oUip = (mo >> 9) & 1; oV = (mo >> 2) & 1;
+      oVjp = (m[1] >> 2) & 1; oEjp = (m[1] >> 3) & 1; oEjm = (m[3] >> 3) & 1;
+      oEipp = (__shfl_down_sync(FULLM, mo, 1) >> 11) & 1;
+      oEjpp = (m[0] >> 3) & 1;
+    }
+    const float Do = D[2], Dip = vdown(Do, 1), Djp = D[1], Djm = D[3];
+    const float ro = rD[2], rip = vdown(ro, 1), rjp = rD[1], rjm = rD[3];
+    const float uip = vdown(u[2], 1), vjp = v[1];
+    const float *r = rr[2], *rp = rr[1];
+    const float cv = r[RT_CV], cvp = rp[RT_CV];
+    auto avg2 = [](float a, unsigned oa, float b, unsigned ob) {
+      const unsigned c = FAST ? 2 : oa + ob;
+      return c == 0 ? 0.f : ((oa ? a : 0.f) + (ob ? b : 0.f)) * (c == 2 ? 0.5f : 1.f);
+    };
+    const float huip = avg2(Dip, oEip, Do, oE);
+    const float c8 = oUip ? r[RT_D8] : 0.f;
+    // Advective fluxes through the east and north faces of every lane's
+    // cell, and the diffusive flux through the east face.  The west face
+    // of a cell is the east face of the lane below it, the south face the
+    // north face of the previous output row.
+    const V ch = chs[2], chjp = chs[1], chjm = chs[3];
+    const V chip = vdown(ch, 1), chim = vup(ch), chrr = FLUX ? vdown(ch, 2) : vb<V>(0.f);
+    const V mC = vmul(ch, vb<V>(-ro));  // -C
+    const V fxe = face_flux<FAST, FLUX>(uip, chim, ch, chip, chrr, oUip, oEim, oE, oEip, oEipp);
+    const V fyn = face_flux<FAST, FLUX>(cvp * vjp, chjm, ch, chjp, chs[0], oVjp, oEjm, oE, oEjp, oEjpp);
+    const V fys = fyp;
+    fyp = fyn;
+    const V dxe = vmul(vmul(vfma(chip, vb<V>(rip), mC), vb<V>(huip)), vb<V>(c8));
+    const V fxw = vup(fxe), dxw = vup(dxe);
+    if (!upd) return;
+    const int ko = gi + off[2];
+    const float hv = avg2(Do, oE, Djm, oEjm), hvjp = avg2(Djp, oEjp, Do, oE);
+    const float c10 = oVjp ? cvp * r[RT_D10] : 0.f, c11 = oV ? cv * r[RT_D10] : 0.f;
+    V g = vfma(vsub(fxw, fxe), vb<V>(r[RT_RDL]), vmul(vsub(fys, fyn), vb<V>(r[RT_RDT])));
+    if (!FAST && FLUX == 1 && !oE) g = vb<V>(0.f);
+    if (oE) {
+      V kappa, gam, sum = vsub(dxe, dxw);
+      sum = vfma(vmul(vfma(chjp, vb<V>(rjp), mC), vb<V>(hvjp)), vb<V>(c10), sum);
+      sum = vfma(vmul(vfma(chjm, vb<V>(rjm), mC), vb<V>(hv)), vb<V>(c11), sum);
+#pragma unroll
+      for (int q = 0; q < NT; q++) {
+        half(kappa, q) = p.t[q].kappa;
+        half(gam, q) = p.t[q].gamma ? p.t[q].gamma[ko] : p.t[q].gamma_s;
+      }
+      // kappa (diffusion) - gamma D (C - C0) + C Fe
+      V rest = vfma(kappa, sum, vmul(vmul(gam, vb<V>(Do)), vadd(mC, pc0)));
+      if (p.Fe) rest = vfma(mC, vb<V>(-p.Fe[ko]), rest);
+      g = vadd(g, rest);
+    }
+    const V x = vfma(vb<V>(p.ab2), g, vfma(vb<V>(p.ab0), pg1, vmul(vb<V>(p.ab1), pg2)));
+    V nh, nl, ndp;
+#pragma unroll
+    for (int q = 0; q < NT; q++) half(ndp, q) = p.decay ? -(p.t[q].dp ? p.t[q].dp[ko] : p.t[q].dp_s) : 0.f;
+    comp_update(chh[2], chl[2], vb<V>(p.dt), x, p.decay != 0, ndp, nh, nl);
+#pragma unroll
+    for (int q = 0; q < NT; q++) {
+      p.t[q].G3[ko] = half(g, q);
+      p.t[q].chn[ko] = half(nh, q);
+      p.t[q].cln[ko] = half(nl, q);
+    }
+  };
 
   for (; J < jend; J++) {
 #pragma unroll
-    for (int a = 4; a > 0; a--) {
+    for (int a = 3; a > 0; a--) {
       m[a] = m[a - 1];
       D[a] = D[a - 1];
       rD[a] = rD[a - 1];
-#pragma unroll
-      for (int q = 0; q < NT; q++) chs[q][a] = chs[q][a - 1];
+      chs[a] = chs[a - 1];
     }
 #pragma unroll
     for (int a = 2; a > 0; a--) {
@@ -156,131 +305,32 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : (NT <= 3 ? 4 : 3)) k_trc32(
       v[a] = v[a - 1];
       off[a] = off[a - 1];
       rr[a] = rr[a - 1];
-#pragma unroll
-      for (int q = 0; q < NT; q++) {
-        if (!RELOAD) {
-          chh[q][a] = chh[q][a - 1];
-          chl[q][a] = chl[q][a - 1];
-        }
-      }
+      chh[a] = chh[a - 1];
+      chl[a] = chl[a - 1];
     }
     m[0] = n1.m; D[0] = n1.D; rD[0] = rthick(n1.D); u[0] = n1.u; v[0] = n1.v; off[0] = n1.off; rr[0] = n1.rows;
-#pragma unroll
-    for (int q = 0; q < NT; q++) {
-      if (!RELOAD) {
-        chh[q][0] = n1.h[q];
-        chl[q][0] = n1.l[q];
-      }
-      chs[q][0] = n1.h[q] + n1.l[q];
-    }
+    chh[0] = n1.h;
+    chl[0] = n1.l;
+    chs[0] = vadd(n1.h, n1.l);
     n1 = n2;
     if (J + 2 < jend) load(J + 2, n2);
     if (PF) {
-      if (J + 4 < jend) {  // rows two beyond the one just loaded
-        const int k4 = gi + nx * wr(J + 4, ny);
-        prefetch_l2(p.mask16 + k4);
-        prefetch_l2(p.He + k4);
-        if (p.nl) prefetch_l2(p.eta + k4);
-        prefetch_l2(p.u + k4);
-        prefetch_l2(p.v + k4);
-#pragma unroll
-        for (int q = 0; q < NT; q++) {
-          prefetch_l2(p.t[q].ch + k4);
-          prefetch_l2(p.t[q].cl + k4);
-        }
-      }
-      if (store_lane && J >= ry0 && J < ylast) {  // update inputs of output row J (loaded at J + 1)
-        const int k0 = gi + off[0];
-#pragma unroll
-        for (int q = 0; q < NT; q++) {
-          prefetch_l2(p.t[q].G1 + k0);
-          prefetch_l2(p.t[q].G2 + k0);
-          prefetch_l2(p.t[q].C0 + k0);
-        }
-      }
+      const bool want = pfp && (pfi ? J >= ry0 && J < ylast : J + 4 < jend);
+      if (want) prefetch_l2(pfp + (size_t)(unsigned)(pfi ? off[0] : nx * wr(J + 4, ny)) * pfs);
     }
-
-    const int o = J - 2;
     // row ry0 - 1 only forms its north faces (the south faces of row ry0)
-    if (o >= ry0 - 1) {  // uniform across the warp
-      const bool upd = store_lane && o >= ry0 && o < ny;
-      // masks of row o and its neighbours
-      const unsigned mo = m[2];
-      const unsigned oE = (mo >> 3) & 1, oEim = (mo >> 7) & 1, oEip = (mo >> 11) & 1;
-      const unsigned oUip = (mo >> 9) & 1, oV = (mo >> 2) & 1;
-      const unsigned oVjp = (m[1] >> 2) & 1, oEjp = (m[1] >> 3) & 1, oEjm = (m[3] >> 3) & 1;
-      const unsigned oEipp = (__shfl_down_sync(FULLM, mo, 1) >> 11) & 1;
-      const unsigned oEjpp = (m[0] >> 3) & 1;
-      const float Do = D[2], Dip = __shfl_down_sync(FULLM, Do, 1);
-      const float Djp = D[1], Djm = D[3];
-      const float ro = rD[2], rip = __shfl_down_sync(FULLM, ro, 1);
-      const float rjp = rD[1], rjm = rD[3];
-      const float uip = __shfl_down_sync(FULLM, u[2], 1), vjp = v[1];
-      const float *r = rr[2], *rp = rr[1];
-      const float cv = r[RT_CV], cvp = rp[RT_CV];
-      auto avg2 = [](float a, unsigned oa, float b, unsigned ob) {
-        unsigned c = oa + ob;
-        return c == 0 ? 0.f : ((oa ? a : 0.f) + (ob ? b : 0.f)) * (c == 2 ? 0.5f : 1.f);
-      };
-      const float huip = avg2(Dip, oEip, Do, oE);
-      const float c8 = oUip * r[RT_D8];
-      // Advective fluxes through the east and north faces of every lane's
-      // cell, and the diffusive flux through the east face.  The west face
-      // of a cell is the east face of the lane below it, the south face the
-      // north face of the previous output row: the same operands in the same
-      // order, so the same bits as forming them again (and one call site, so
-      // one rounding of the contracted arithmetic).
-      float fxe[NT], fxw[NT], fyn[NT], fys[NT], dxe[NT], dxw[NT];
-#pragma unroll
-      for (int q = 0; q < NT; q++) {
-        const float ch = chs[q][2], chip = __shfl_down_sync(FULLM, ch, 1), chim = __shfl_up_sync(FULLM, ch, 1);
-        const float chrr = FLUX ? __shfl_down_sync(FULLM, ch, 2) : 0.f;
-        const float chjp = chs[q][1], chjm = chs[q][3];
-        fxe[q] = oUip * uip * face(FLUX, uip, chim, ch, chip, chrr, oEim, oE, oEip, oEipp);
-        fyn[q] = oVjp * cvp * vjp * face(FLUX, vjp, chjm, ch, chjp, chs[q][0], oEjm, oE, oEjp, oEjpp);
-        fys[q] = fyp[q];
-        fyp[q] = fyn[q];
-        dxe[q] = huip * (chip * rip - ch * ro) * c8;
-        fxw[q] = __shfl_up_sync(FULLM, fxe[q], 1);
-        dxw[q] = -__shfl_up_sync(FULLM, dxe[q], 1);
-      }
-      if (upd) {
-        const int ko = gi + off[2];
-        const float rdl = r[RT_RDL], rdt = r[RT_RDT];
-        const float hv = avg2(Do, oE, Djm, oEjm), hvjp = avg2(Djp, oEjp, Do, oE);
-        const float Fe = p.Fe ? p.Fe[ko] : 0.f;
-        const float c10 = oVjp * cvp * r[RT_D10], c11 = -(float)oV * cv * r[RT_D10];
-#pragma unroll
-        for (int q = 0; q < NT; q++) {
-          const auto &t = p.t[q];
-          const float ch = chs[q][2], chjp = chs[q][1], chjm = chs[q][3];
-          float g = rdl * (fxw[q] - fxe[q]) + rdt * (fys[q] - fyn[q]);
-          if (FLUX == 1 && !oE) g = 0.f;
-          if (oE) {
-            const float C = ch * ro;
-            const float diff =
-                t.kappa * (dxe[q] + dxw[q] + hvjp * (chjp * rjp - C) * c10 + hv * (C - chjm * rjm) * c11);
-            const float gam = t.gamma ? t.gamma[ko] : t.gamma_s;
-            g += diff - gam * Do * (C - pc0[q]) + C * Fe;
-          }
-          t.G3[ko] = g;
-          const float inc = p.dt * (p.ab0 * pg1[q] + p.ab1 * pg2[q] + p.ab2 * g);
-          float nh, nl;
-          comp_update(RELOAD ? t.ch[ko] : chh[q][2], RELOAD ? t.cl[ko] : chl[q][2], inc, t.dp ? t.dp[ko] : t.dp_s,
-                      nh, nl);
-          t.chn[ko] = nh;
-          t.cln[ko] = nl;
-        }
-      }
+    if (J - 2 >= ry0 - 1) {  // uniform across the warp
+      if (__all_sync(FULLM, (m[0] & m[1] & m[2] & m[3] & 0xfffu) == 0xfffu)) body(std::true_type{});
+      else body(std::false_type{});
     }
     // update inputs of the next output row (J - 1)
     if (store_lane && J - 1 >= ry0 && J - 1 < ylast) {
       const int kn = gi + off[1];
 #pragma unroll
       for (int q = 0; q < NT; q++) {
-        pg1[q] = p.t[q].G1[kn];
-        pg2[q] = p.t[q].G2[kn];
-        pc0[q] = p.t[q].C0[kn];
+        half(pg1, q) = p.t[q].G1[kn];
+        half(pg2, q) = p.t[q].G2[kn];
+        half(pc0, q) = p.t[q].C0[kn];
       }
     }
   }
@@ -335,9 +385,7 @@ static int trc_resident_nt(const TrcP &p) {
 static void trc_launch(const TrcP &p, int S, cudaStream_t st) {
   switch (p.ntr) {
     case 1: trc_launch_nt<1>(p, S, st); break;
-    case 2: trc_launch_nt<2>(p, S, st); break;
-    case 3: trc_launch_nt<3>(p, S, st); break;
-    default: trc_launch_nt<4>(p, S, st); break;
+    default: trc_launch_nt<2>(p, S, st); break;
   }
 }
 
@@ -345,9 +393,7 @@ static void trc_launch(const TrcP &p, int S, cudaStream_t st) {
 static int trc_resident(const TrcP &p) {
   switch (p.ntr) {
     case 1: return trc_resident_nt<1>(p);
-    case 2: return trc_resident_nt<2>(p);
-    case 3: return trc_resident_nt<3>(p);
-    default: return trc_resident_nt<4>(p);
+    default: return trc_resident_nt<2>(p);
   }
 }
 
@@ -390,7 +436,7 @@ __global__ void k_f64_to_f32(const double *a, float *b, size_t n) {
 
 struct Trc32State {
   std::vector<swm::Tracer32> t;
-  int warp_rows = 0;  // rows per warp of the tracer kernel (0: not tuned yet)
+  int warp_rows[swm::TRC32_MAX] = {};  // rows per warp by tracers per launch (0: not tuned yet)
   float *rows = nullptr;
   float *u = nullptr, *v = nullptr, *eta = nullptr;  // frozen-flow copies
   bool ready = false;
@@ -526,6 +572,7 @@ int trc32_step(swm_gpu_ctx *c, int64_t itt) {
   for (size_t t0 = 0; t0 < s->t.size(); t0 += TRC32_MAX) {
     p.ntr = (int)std::min(s->t.size() - t0, (size_t)TRC32_MAX);
     p.pf = trc_prefetch(c->n, p.ntr);
+    p.decay = 0;
     for (int q = 0; q < p.ntr; q++) {
       const Tracer32 &T = s->t[t0 + q];
       auto &d = p.t[q];
@@ -533,9 +580,15 @@ int trc32_step(swm_gpu_ctx *c, int64_t itt) {
       d.G1 = T.G[T.g0]; d.G2 = T.G[(T.g0 + 1) % 3]; d.G3 = T.G[(T.g0 + 2) % 3];
       d.C0 = T.C0; d.gamma = T.gamma; d.dp = T.dp;
       d.gamma_s = T.gamma_s; d.dp_s = T.dp_s; d.kappa = T.kappa;
+      p.decay |= T.dp != nullptr || T.dp_s != 0.f;
     }
-    if (!s->warp_rows) s->warp_rows = trc_tune_rows(c, p);
-    trc_launch(p, s->warp_rows, c->stream);
+    int &rows = s->warp_rows[p.ntr - 1];
+    if (!rows) {  // timed on the first step of this kind; steps being captured go untimed
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      SWM_CK(cudaStreamIsCapturing(c->stream, &cap));
+      if (cap == cudaStreamCaptureStatusNone) rows = trc_tune_rows(c, p);
+    }
+    trc_launch(p, rows ? rows : 2 * TRC_ROWS, c->stream);
     c->launches++;
   }
   SWM_CK(cudaGetLastError());
