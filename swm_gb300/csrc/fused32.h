@@ -3,6 +3,7 @@
 #include <functional>
 #include <vector>
 #include "ctx.h"
+#include "pdl.cuh"
 
 namespace swm {
 
@@ -66,14 +67,6 @@ struct F2 {
   __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
 
-// Programmatic dependent launch: a kernel launched with
-// cudaLaunchAttributeProgrammaticStreamSerialization may start before its
-// predecessor on the stream has finished; grid_dep_wait() returns once the
-// predecessor has completed and its writes are visible (at once for a kernel
-// launched the ordinary way).  grid_dep_trigger() lets the successor launch.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // ask L2 for the line holding a (no register is written, nothing waits)
 __device__ __forceinline__ void prefetch_l2(const void *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
@@ -121,21 +114,6 @@ struct MonitorStep {
 // blocks) into out[3]
 void march_integrals_final(const double *partial, int nb, double G, double *out, cudaStream_t st);
 
-// cudaLaunchKernelEx with programmatic stream serialisation (see grid_dep_wait)
-template <typename... KArgs, typename... Args>
-cudaError_t launch_programmatic(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 // the step kernel's tiles (device) and blocks
 struct MarchGrid {
   const int2 *tiles;
