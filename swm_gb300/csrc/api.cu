@@ -673,8 +673,9 @@ static const double *field_ptr(swm_gpu_ctx *c, int f, double **wptr) {
 
 // device copy of a field as of the current state (fused paths: the FP64
 // field, or the state and the diagnostics, are formed from the FP32 pair state
-// first; converting the one field asked for and not all six took the fields of
-// a 256-member ensemble from 26 to OUT1 ms)
+// first; converting the one field asked for and not all six, and writing it
+// into a pinned array without a copy, took the fields of a 256-member ensemble
+// from 26 to 13 ms)
 static int field_device(swm_gpu_ctx *c, int f, const double **out) {
   if (c->cfg.path != SWM_PATH_PLAIN_FP64 && c->stage >= 5 && c->fused) {
     const bool diag = f >= SWM_F_D && f <= SWM_F_MV;
@@ -724,9 +725,21 @@ extern "C" {
 int swm_gpu_get_field_async(swm_gpu_ctx *c, int f, double *out, int64_t *ticket) {
   SWM_ON_DEVICE(c ? c->device : -1);
   SWM_REQUIRE(c && c->stage >= 1 && out && ticket, "swm_gpu_get_field_async: bad arguments");
-  const double *p = nullptr;
-  TRY(field_device(c, f, &p));
-  SWM_CK(cudaMemcpyAsync(out, p, c->n * 8, cudaMemcpyDeviceToHost, c->stream));
+  // a small field of the pair state goes straight into a pinned array: the
+  // kernel that joins its words writes them there, and no copy follows.  A copy
+  // costs the host about 6 us; above a megabyte the copy engine moves the
+  // field beside other kernels, where a kernel's writes hold SMs for as long
+  // (8.4 MB fields of a 1025^2 basin, 96 steps and three fields: 2.62 ms with
+  // copies, 2.67 without)
+  double *view = c->cfg.path == SWM_PATH_FUSED_FP32C && c->n * 8 <= ((size_t)1 << 20) ? mapped_view(out) : nullptr;
+  if (view && mapped_view(out + c->n - 1) != view + c->n - 1) view = nullptr;  // pinned to its end
+  bool done = false;
+  if (view && c->stage >= 5) TRY(fused_sync_field(c, f, view, &done));
+  if (!done) {
+    const double *p = nullptr;
+    TRY(field_device(c, f, &p));
+    SWM_CK(cudaMemcpyAsync(out, p, c->n * 8, cudaMemcpyDeviceToHost, c->stream));
+  }
   return async_record(c, ticket);
 }
 

@@ -215,7 +215,8 @@ int fused_step(swm_gpu_ctx *c, int64_t itt);
 int fused_sync_state(swm_gpu_ctx *c);    // FP32 pair state -> FP64 buffers
 int fused_load_state(swm_gpu_ctx *c);    // FP64 buffers -> FP32 pair state
 int fused_load_field(swm_gpu_ctx *c, int field);  // the same for one of u, v, eta
-int fused_sync_field(swm_gpu_ctx *c, int field);  // fused_sync_state for what one field's read needs
+// fused_sync_state for what one field's read needs, or that field straight into `to`
+int fused_sync_field(swm_gpu_ctx *c, int field, double *to = nullptr, bool *done = nullptr);
 int fused_refresh_wind(swm_gpu_ctx *c, int id);  // stream id's record changed
 int stream_rows(swm_gpu_ctx *c, int id, const double *r1, const double *r2, const double *d1);
 int integrals_to(swm_gpu_ctx *c, double *dst, double **where);  // dst: device or host-mapped

@@ -286,10 +286,12 @@ int fused_load_field(swm_gpu_ctx *c, int field) {
   return SWM_GPU_OK;
 }
 
-// one field of the pair state, or its newest increment, -> the FP64 buffer
-// that swm_gpu_get_field reads (other fields need none)
-int fused_sync_field(swm_gpu_ctx *c, int field) {
+// one field of the pair state, or its newest increment, -> `to`, or where that
+// is null the FP64 buffer that swm_gpu_get_field reads (other fields need
+// none); *done (may be null): the field was one of these
+int fused_sync_field(swm_gpu_ctx *c, int field, double *to, bool *done) {
   FusedState *f = c->fused;
+  if (done) *done = false;
   if (!f || !f->ready || !f->comp) return SWM_GPU_OK;
   const int a = f->n0, g = (f->g0 + 1) % 3, cg = (c->g0 + 1) % 3;
   const float *hi = nullptr, *lo = nullptr;
@@ -303,7 +305,8 @@ int fused_sync_field(swm_gpu_ctx *c, int field) {
     case SWM_F_GETA: hi = f->Ge[g]; dst = c->Ge[cg]; break;
     default: return SWM_GPU_OK;
   }
-  k_join<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(hi, lo, dst, c->n);
+  k_join<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(hi, lo, to ? to : dst, c->n);
+  if (done) *done = true;
   c->launches++;
   SWM_CK(cudaGetLastError());
   return SWM_GPU_OK;

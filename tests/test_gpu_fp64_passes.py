@@ -159,3 +159,26 @@ def test_tracer_steps_replayed(shape, flux):
                 g.advance(itt)
         late.append(g.tracer_field(0, 'CH'))
     assert np.array_equal(*late)
+
+
+@pytest.mark.parametrize('shape', [(77, 41), (511, 255), (512, 256)])   # either side of a megabyte
+def test_async_fields_pinned_and_pageable(shape):
+    """A field of the pair state read into a pinned array (a small one is
+    written there by the joining kernel), a pageable one (copied) and by the
+    blocking call is the same, of the state when it was asked for."""
+    import torch
+    case = make(shape, 'laplacian')
+    g = GpuModel('fused_fp32c')
+    run_case(case, g, nsteps=10, with_diag=False)
+    now = {f: g.field(f) for f in ('u', 'v', 'eta', 'G_u', 'D')}
+    shape = now['u'].shape
+    got = {}
+    for f in now:
+        pinned, plain = torch.empty(shape, dtype=torch.float64).pin_memory().numpy(), np.empty(shape)
+        got[f] = (pinned, plain, g.field_async(f, pinned), g.field_async(f, plain))
+    g.run(10, 12)
+    for f, (pinned, plain, t, s) in got.items():
+        g.wait(t)
+        g.wait(s)
+        assert np.array_equal(pinned, now[f]) and np.array_equal(plain, now[f]), f
+    g.close()
