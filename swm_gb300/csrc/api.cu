@@ -38,6 +38,10 @@ swm::Dev swm_gpu_ctx::dev() const {
     d.rimpl[q] = rimpl[q];
     d.impl_how[q] = pdiv ? impl_how[q] : IMPL_DIVIDE;
   }
+  for (int q = 0; q < 2; q++) {
+    d.rdepth[q] = rdepth[q];
+    d.depth_how[q] = pdiv ? depth_how[q] : IMPL_DIVIDE;
+  }
   for (int q = 0; q < 4; q++) {
     d.ocean[q] = d_ocean[q];
     d.cosl[q] = d_cos[q];
@@ -183,7 +187,7 @@ int swm_gpu_destroy(swm_gpu_ctx *c) {
   for (int q = 0; q < 3; q++) { F(c->Gu[q]); F(c->Gv[q]); F(c->Ge[q]); F(c->impl[q]); F(c->glin[q]); F(c->F[q]); F(c->Fc[q]); }
   F(c->edens); F(c->pot); F(c->zeta); F(c->mu); F(c->mv); F(c->pll); F(c->plt); F(c->lmu); F(c->lmv);
   F(c->latp[0]); F(c->latp[1]); F(c->latuv); F(c->prow); F(c->pk); F(c->rimpl[0]); F(c->rimpl[1]);
-  F(c->rimpl[2]); F(c->pdiv_flags); F(c->ubs); F(c->vbs); F(c->zbs); F(c->trc_coeff); F(c->rows_buf); F(c->march_tiles);
+  F(c->rimpl[2]); F(c->pdiv_flags); F(c->rdepth[0]); F(c->rdepth[1]); F(c->ubs); F(c->vbs); F(c->zbs); F(c->trc_coeff); F(c->rows_buf); F(c->march_tiles);
   for (auto &s : c->streams) { F(s.d1); F(s.d2); F(s.rec[0]); F(s.rec[1]); }
   for (auto &t : c->tracers) {
     F(t.CH[0]); F(t.CH[1]); F(t.G[0]); F(t.G[1]); F(t.G[2]); F(t.C); F(t.C0); F(t.gamma); F(t.impl);
@@ -806,8 +810,12 @@ int swm_gpu_set_field(swm_gpu_ctx *c, int f, const double *in) {
   SWM_CK(cudaStreamSynchronize(c->stream));
   c->stress_ready = false;  // the plain path forms the stress of the next step again
   if (c->cfg.path != SWM_PATH_PLAIN_FP64 && c->stage >= 5 && f <= SWM_F_ETA) TRY(fused_load_field(c, f));
-  if (f == SWM_F_IMPL_U || f == SWM_F_IMPL_V || f == SWM_F_IMPL_ETA) {
-    c->pdiv_ready = false;  // the plain path's reciprocals of the damping factors are formed again
+  // the plain path forms its reciprocals of the damping factors again, in the
+  // linear modes those of the thickness and the potential vorticity too
+  const bool linear = c->cfg.mode == SWM_MODE_LIN_REST || c->cfg.mode == SWM_MODE_LIN_MEAN;
+  if (f == SWM_F_IMPL_U || f == SWM_F_IMPL_V || f == SWM_F_IMPL_ETA || (linear && f > SWM_F_ETA)) {
+    c->pdiv_ready = false;
+    c->pot_ready = false;
     invalidate_graph(c);
   }
   return SWM_GPU_OK;

@@ -106,6 +106,8 @@ struct Dev {
   const PlainRow *prow;     // per row
   const PlainConst *pk;     // of the whole grid
   const double *rimpl[3];   // 1 / impl_u, _v, _eta
+  int depth_how[2];         // IMPL_*: how the mixing of u, v is divided by the thickness
+  const double *rdepth[2];  // 1 / Du, 1 / Dv (linear modes)
   const int8_t *ocean[4];
   const double *cosl[4], *tanl[4], *f[4];
   double *Hg[4];  // H, H_u, H_v, H_eta on the device (H/H_u/H_v overwritten at itt=0 in linear modes)
@@ -158,7 +160,10 @@ struct swm_gpu_ctx {
   double *rimpl[3] = {};
   unsigned *pdiv_flags = nullptr;
   int impl_how[3] = {};
+  double *rdepth[2] = {};
+  int depth_how[2] = {};
   bool pdiv = false, pdiv_ready = false;
+  bool pot_ready = false;     // linear modes: the potential vorticity is that of the grid's fields
   bool stress_ready = false;  // pll, plt (biharmonic: bh[0], bh[1]) are those of the current state (plain path)
   double *impl[3] = {}, *gsq[2] = {}, *glin[3] = {};
   double *F[3] = {}, *Fc[3] = {};

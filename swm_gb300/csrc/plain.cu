@@ -116,12 +116,15 @@ __global__ void k_plain_rows(Dev d, PlainRow *rows) {
   P.zl = d.lbc / (d.A * d.cosl[GH][j] * d.dLambda);
 }
 
-// divisors of the whole grid: dLambda, dTheta, A dTheta, and the damping
-// factor of u, v, eta where it is the same everywhere
+// divisors of the whole grid: dLambda, dTheta, A dTheta, the damping factor of
+// u, v, eta where it is the same everywhere, and in the linear modes the
+// thickness at the u and v points where that is (its value at ku, kv)
 struct PlainConst {
-  FixedDiv dL, dT, AdT, impl[3];
+  FixedDiv dL, dT, AdT, impl[3], D[2];
 };
-__global__ void k_plain_const(Dev d, PlainConst *k) {
+__global__ void k_plain_const(Dev d, PlainConst *k, size_t ku, size_t kv) {
+  k->D[0] = fixed_div(d.Du[ku]);
+  k->D[1] = fixed_div(d.Dv[kv]);
   k->dL = fixed_div(d.dLambda);
   k->dT = fixed_div(d.dTheta);
   k->AdT = fixed_div(d.A * d.dTheta);
@@ -144,6 +147,27 @@ __global__ void k_plain_impl(Dev d, double *r0, double *r1, double *r2, unsigned
     r[f][k] = 1. / x;
     if (!div_rn_range(x)) m |= 1u << f;
     if (__double_as_longlong(x) != __double_as_longlong(impl[f][0])) m |= 8u << f;
+  }
+  if (m) atomicOr(flags, m);
+}
+
+// the thickness at the ocean u and v points in the linear modes, where it does
+// not change: 1 / D per point, and as above bits 6, 7 (out of range) and 8, 9
+// (not the value at ku, kv)
+__global__ void k_plain_depth(Dev d, double *r0, double *r1, size_t ku, size_t kv, unsigned *flags) {
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= (size_t)d.nx * d.ny) return;
+  const double *D[2] = {d.Du, d.Dv};
+  const int8_t *o[2] = {d.ocean[GU], d.ocean[GV]};
+  double *r[2] = {r0, r1};
+  const size_t at[2] = {ku, kv};
+  unsigned m = 0;
+  for (int f = 0; f < 2; f++) {
+    const double x = D[f][k];
+    r[f][k] = 1. / x;
+    if (o[f][k] != 1) continue;
+    if (!div_rn_range(x)) m |= 64u << f;
+    if (__double_as_longlong(x) != __double_as_longlong(D[f][at[f]])) m |= 256u << f;
   }
   if (m) atomicOr(flags, m);
 }
@@ -260,6 +284,7 @@ __global__ void k_latmix_uv1(Dev d, const double *__restrict__ tab, const double
 // what k_plain_diag forms besides the diagnostics
 struct DiagJobs {
   int interp;         // the thicknesses on H, u and v points (and D in FULLY_NONLINEAR)
+  int pot;            // the potential vorticity (in the linear modes it does not change)
   int forcing;        // reset the forcing and add the wind streams below
   int nwind;
   int merid[2];       // their component
@@ -320,8 +345,10 @@ __global__ void __launch_bounds__(256) k_plain_diag(Dev d, DiagJobs w) {
     d.zeta[k] = zeta;
   }
   if (d.mode != SWM_MODE_NONE) {
-    const double pD = at_least_eps(Dh), fH = d.f[GH][j];
-    d.pot[k] = (nl ? fH + zeta : (d.mode == SWM_MODE_LIN_MEAN ? fH + d.zbs[k] : fH)) / pD;
+    if (w.pot) {
+      const double pD = at_least_eps(Dh), fH = d.f[GH][j];
+      d.pot[k] = (nl ? fH + zeta : (d.mode == SWM_MODE_LIN_MEAN ? fH + d.zbs[k] : fH)) / pD;
+    }
     if (e0) {
       const size_t ku = IDX(ip1(i, d.nx), j), kv = IDX(i, ip1(j, d.ny));
       double E = d.G * eta;
@@ -385,6 +412,12 @@ __global__ void __launch_bounds__(256) k_plain_step(Dev d, const double *__restr
   const double *T = tuv + (size_t)LATUV_N * j;
   const double u = d.u0[k], v = d.v0[k];
   double ge, gu, gv;
+  // f: 0 by the thickness at the u point, 1 at the v point
+  auto by_depth = [&](double x, int f, const double *D) {
+    if (d.depth_how[f] == IMPL_SAME) return div_fixed(x, K.D[f]);
+    if (d.depth_how[f] == IMPL_FAST) return div_fast(x, D[k], d.rdepth[f][k]);
+    return x / D[k];
+  };
   if (d.ocean[GE][k] == 1) {  // continuity
     const double *cV = d.cosl[GV];
     auto dL = [&](double x) { return d.pdiv ? div_fixed(x, K.dL) : x / d.dLambda; };
@@ -417,7 +450,7 @@ __global__ void __launch_bounds__(256) k_plain_step(Dev d, const double *__restr
       g = g - q;
     }
     if (tuv) {
-      const double l = mix_u(d, T, d.pll, d.plt, i, j) / d.Du[k];
+      const double l = by_depth(mix_u(d, T, d.pll, d.plt, i, j), 0, d.Du);
       d.lmu[k] = l;
       g = g + l;
     }
@@ -439,7 +472,7 @@ __global__ void __launch_bounds__(256) k_plain_step(Dev d, const double *__restr
       g = g - q;
     }
     if (tuv) {
-      const double l = mix_v(d, T, d.pll, d.plt, i, j) / d.Dv[k];
+      const double l = by_depth(mix_v(d, T, d.pll, d.plt, i, j), 1, d.Dv);
       d.lmv[k] = l;
       g = g + l;
     }
@@ -570,6 +603,7 @@ int plain_diagnostics(swm_gpu_ctx *c, int64_t itt) {
   const int mode = c->cfg.mode;
   DiagJobs w = {};
   w.interp = mode == SWM_MODE_NONLINEAR || mode == SWM_MODE_NONE || itt == 0;
+  w.pot = 1;
   LAUNCH(k_plain_diag, c->dev(), w);
   SWM_CK(cudaGetLastError());
   return SWM_GPU_OK;
@@ -658,7 +692,21 @@ int plain_prepare(swm_gpu_ctx *c) {
     SWM_CK(cudaMemsetAsync(c->pdiv_flags, 0, sizeof(unsigned), c->stream));
     const Dev d = c->dev();
     k_plain_rows<<<(c->ny + 127) / 128, 128, 0, c->stream>>>(d, c->prow);
-    k_plain_const<<<1, 1, 0, c->stream>>>(d, c->pk);
+    // the thickness stays in the linear modes: divisions by it as by the others
+    const bool linear = c->cfg.mode == SWM_MODE_LIN_REST || c->cfg.mode == SWM_MODE_LIN_MEAN;
+    size_t at[2] = {0, 0};
+    for (int f = 0; f < 2; f++) {
+      const std::vector<int8_t> &o = c->hg.ocean[f ? GV : GU];
+      while (at[f] + 1 < n && !o[at[f]]) at[f]++;
+    }
+    k_plain_const<<<1, 1, 0, c->stream>>>(d, c->pk, at[0], at[1]);
+    if (linear) {
+      for (int f = 0; f < 2; f++)
+        if (!c->rdepth[f]) SWM_CK(cudaMalloc((void **)&c->rdepth[f], n * sizeof(double)));
+      k_plain_depth<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(d, c->rdepth[0], c->rdepth[1], at[0], at[1],
+                                                                     c->pdiv_flags);
+      c->launches++;
+    }
     k_plain_impl<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(d, c->rimpl[0], c->rimpl[1], c->rimpl[2],
                                                                   c->pdiv_flags);
     c->launches += 3;
@@ -668,6 +716,8 @@ int plain_prepare(swm_gpu_ctx *c) {
     SWM_CK(cudaStreamSynchronize(c->stream));
     for (int f = 0; f < 3; f++)
       c->impl_how[f] = !((fl >> (3 + f)) & 1) ? IMPL_SAME : ((fl >> f) & 1 ? IMPL_DIVIDE : IMPL_FAST);
+    for (int f = 0; f < 2; f++)
+      c->depth_how[f] = !linear || ((fl >> (6 + f)) & 1) ? IMPL_DIVIDE : ((fl >> (8 + f)) & 1 ? IMPL_FAST : IMPL_SAME);
     c->pdiv = true;
     c->pdiv_ready = true;
   }
@@ -709,6 +759,7 @@ int plain_advance(swm_gpu_ctx *c, int64_t itt) {
   DiagJobs w = {};
   w.interp = mode == SWM_MODE_NONLINEAR || mode == SWM_MODE_NONE || itt == 0;
   w.forcing = 1;
+  w.pot = mode == SWM_MODE_NONLINEAR || itt == 0 || !c->pot_ready;
   // up to two wind streams of FULLY_NONLINEAR go with the diagnostics
   // (their stress is divided by the thickness formed there)
   bool others = false;
@@ -727,6 +778,7 @@ int plain_advance(swm_gpu_ctx *c, int64_t itt) {
   LAUNCH(k_plain_diag, c->dev(), w);
   SWM_CK(cudaGetLastError());
   c->stress_ready = c->cfg.lateral_mixing != 0;
+  c->pot_ready = true;
   return others ? plain_streams(c, itt, 0) : SWM_GPU_OK;
 }
 

@@ -182,3 +182,37 @@ def test_async_fields_pinned_and_pageable(shape):
         g.wait(s)
         assert np.array_equal(pinned, now[f]) and np.array_equal(plain, now[f]), f
     g.close()
+
+
+@pytest.mark.parametrize('field', ['H_u', 'H_v', 'H', 'pot', 'impl_u'])
+@pytest.mark.parametrize('depths', ['flat', 'varied'])
+def test_linear_mode_grid_fields_set_between_steps(field, depths):
+    """The linear modes divide by thicknesses that do not change and keep their
+    potential vorticity: a grid field set between steps reaches the steps that
+    follow, replayed or single, as it does in a model that has always formed
+    everything again (set anew before every step)."""
+    case = synthetic.linear_rg(40, 24, nsteps=STEPS)
+    if depths == 'varied':
+        case['config']['H_overwrite'] = 0.0
+        case['H'] = np.where(case['H'] > 0, 150.0 + 100.0 * np.random.default_rng(2).random(case['H'].shape), 0.0)
+    runs = []
+    for mode in ('replayed', 'single', 'anew'):
+        g = GpuModel('plain_fp64')
+        run_case(case, g, nsteps=0, with_diag=False)
+        g.run(0, 20)
+        new = g.field(field)
+        new[5:12, 6:30] *= 1.25
+        g.set_field(field, new)
+        if mode == 'replayed':
+            g.run(20, 20)
+        else:
+            for itt in range(21, 41):
+                if mode == 'anew' and itt > 21:   # the same values: only what is kept is dropped
+                    g.set_field('gamma_lin_u', g.field('gamma_lin_u'))
+                g.step(itt)
+                g.advance(itt)
+        runs.append([g.field(f) for f in ('u', 'v', 'eta', 'pot')])
+        g.close()
+    for other in runs[1:]:
+        for a, b in zip(runs[0], other):
+            assert np.array_equal(a, b)
