@@ -194,6 +194,9 @@ int swm_gpu_destroy(swm_gpu_ctx *c) {
     F(t.uhc); F(t.vhc); F(t.diff);
   }
   for (auto e : c->async_ev) cudaEventDestroy(e);
+  if (c->fork) cudaEventDestroy(c->fork);
+  if (c->join) cudaEventDestroy(c->join);
+  if (c->branch) cudaStreamDestroy(c->branch);
   cudaStreamDestroy(c->stream);
   delete c;
   return SWM_GPU_OK;
@@ -403,16 +406,42 @@ int swm_gpu_initial_conditions(swm_gpu_ctx *c, const double *eta, const double *
   return SWM_GPU_OK;
 }
 
+// A captured step with FP64 tracers: their increment and update read the same
+// old level as the flow's step and write fields of their own, so they go to a
+// branch beside it, with the fluxes of the last advance (which read the mass
+// fluxes and concentrations that the next advance rewrites: the branch joins
+// before it).
+static int step_branched(swm_gpu_ctx *c, int64_t itt) {
+  SWM_CK(cudaEventRecord(c->fork, c->stream));
+  SWM_CK(cudaStreamWaitEvent(c->branch, c->fork, 0));
+  TRY(tracer_step(c, itt, c->branch));
+  if (c->flux_due) TRY(tracer_flux(c, c->branch));
+  c->flux_due = false;
+  TRY(plain_step(c, itt));
+  SWM_CK(cudaEventRecord(c->join, c->branch));
+  SWM_CK(cudaStreamWaitEvent(c->stream, c->join, 0));
+  return SWM_GPU_OK;
+}
+
+// a tracer's part of the advance
+static int tracers_advance(swm_gpu_ctx *c) {
+  TRY(tracer_advance(c));
+  if (c->branching) c->flux_due = true;
+  else TRY(tracer_flux(c, c->stream));
+  return SWM_GPU_OK;
+}
+
 static int swm_step_impl(swm_gpu_ctx *c, int64_t itt) {
   // FP32 tracers read the level the SWM step reads, so they go first
   if (trc32_active(c)) TRY(trc32_step(c, itt));
   if (c->cfg.frozen_flow) {  // prescribed flow: only the tracers step
-    if (!c->tracers.empty() && !trc32_active(c)) TRY(tracer_step(c, itt));
+    if (!c->tracers.empty() && !trc32_active(c)) TRY(tracer_step(c, itt, c->stream));
     return SWM_GPU_OK;
   }
+  if (c->branching) return step_branched(c, itt);
   if (c->cfg.path == SWM_PATH_PLAIN_FP64) TRY(plain_step(c, itt));
   else TRY(fused_step(c, itt));
-  if (!c->tracers.empty() && !trc32_active(c)) TRY(tracer_step(c, itt));
+  if (!c->tracers.empty() && !trc32_active(c)) TRY(tracer_step(c, itt, c->stream));
   return SWM_GPU_OK;
 }
 
@@ -425,7 +454,7 @@ static int swm_advance_impl(swm_gpu_ctx *c, int64_t itt) {
   const bool t32 = trc32_active(c), t64 = !c->tracers.empty() && !t32;
   if (c->cfg.frozen_flow && itt > 0) {  // state, diagnostics and forcing stay
     if (t32) trc32_advance(c);
-    if (t64) TRY(tracer_advance(c));
+    if (t64) TRY(tracers_advance(c));
     return SWM_GPU_OK;
   }
   c->n0 = 1 - c->n0;
@@ -440,7 +469,7 @@ static int swm_advance_impl(swm_gpu_ctx *c, int64_t itt) {
   }
   if (itt > 0) {
     if (t32) trc32_advance(c);
-    if (t64) TRY(tracer_advance(c));
+    if (t64) TRY(tracers_advance(c));
   }
   return SWM_GPU_OK;
 }
@@ -483,12 +512,22 @@ static int graph_capture(swm_gpu_ctx *c, int64_t itt0) {
   }
   const int n0 = c->n0, g0 = c->g0, phase = (int)(c->advances % GRAPH_STEPS);
   const int64_t l0 = c->launches;
+  const bool branch = c->cfg.path == SWM_PATH_PLAIN_FP64 && !c->tracers.empty() && !c->cfg.frozen_flow;
+  if (branch && !c->branch) {
+    SWM_CK(cudaStreamCreateWithFlags(&c->branch, cudaStreamNonBlocking));
+    SWM_CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
+    SWM_CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
+  }
   SWM_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  c->branching = branch;
   int rc = SWM_GPU_OK;
   for (int s = 1; s <= GRAPH_STEPS && rc == SWM_GPU_OK; s++) {
     rc = swm_step_impl(c, itt0 + s);
     if (rc == SWM_GPU_OK) rc = swm_advance_impl(c, itt0 + s);
   }
+  c->branching = false;
+  if (c->flux_due && rc == SWM_GPU_OK) rc = tracer_flux(c, c->stream);
+  c->flux_due = false;
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
   const int64_t nl = c->launches - l0;

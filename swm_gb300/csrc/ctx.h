@@ -189,6 +189,11 @@ struct swm_gpu_ctx {
   int2 *march_tiles = nullptr;       // its tiles, one per warp (device)
   int march_blocks = 0;              // its blocks (tiles / 4)
   cudaGraphExec_t graph = nullptr;  // GRAPH_STEPS captured steps (swm_gpu_run)
+  // while steps with FP64 tracers are captured: the branch that their kernels
+  // go to, its events, and whether an advance's fluxes are still to be issued
+  cudaStream_t branch = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  bool branching = false, flux_due = false;
   int64_t graph_launches = 0;       // kernels in one replay
   int graph_phase = -1;             // rotation phase (advances mod 6) the replay starts from
   swm::Dev dev() const;
@@ -212,8 +217,9 @@ int plain_forcing_update(swm_gpu_ctx *c, int64_t itt, int constant_part);
 int plain_fill(swm_gpu_ctx *c, double *p, double value);
 // tracer.cu
 int tracer_init_coeffs(swm_gpu_ctx *c);
-int tracer_step(swm_gpu_ctx *c, int64_t itt);
+int tracer_step(swm_gpu_ctx *c, int64_t itt, cudaStream_t st);
 int tracer_advance(swm_gpu_ctx *c);
+int tracer_flux(swm_gpu_ctx *c, cudaStream_t st);
 // fused.cu
 int fused_prepare(swm_gpu_ctx *c);
 int fused_step(swm_gpu_ctx *c, int64_t itt);
