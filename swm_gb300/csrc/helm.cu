@@ -318,12 +318,12 @@ __device__ __forceinline__ double widen(float x) {
 // side and iterate, 33 to 41 B a cell, take about 110 us of HBM.
 constexpr int RES_X = 128, RES_ROWS = 32;
 template <typename T>
-__global__ void __launch_bounds__(RES_X) k_h_resid(int nx, int ny, const double *__restrict__ cx,
+__global__ void __launch_bounds__(RES_X) k_h_resid(int nx, int ny, int rows, const double *__restrict__ cx,
                                                    const double *__restrict__ cy, const double *__restrict__ cc,
                                                    const int8_t *__restrict__ mask, const T *__restrict__ rhs,
                                                    const T *__restrict__ psi, double *r, double *partial) {
   __shared__ double red[RES_X / 32];
-  const int i = blockIdx.x * RES_X + threadIdx.x, j0 = blockIdx.y * RES_ROWS, j1 = min(j0 + RES_ROWS, ny);
+  const int i = blockIdx.x * RES_X + threadIdx.x, j0 = blockIdx.y * rows, j1 = min(j0 + rows, ny);
   double acc = 0.;
   if (i < nx) {
     size_t k = (size_t)i + (size_t)nx * j0;
@@ -412,6 +412,7 @@ struct swm_helm {
   double *host = nullptr;  // pinned, 1 double
   float *hinv32 = nullptr, *e32 = nullptr, *r32 = nullptr, *e32b = nullptr;  // e32b: ping-pong of e32
   int tbk = 4;  // sweeps per temporally blocked FP32 launch
+  int sms = 0;
   int8_t *mask = nullptr;
   dim3 blk = dim3(64, 4);
   int64_t launches = 0;
@@ -505,14 +506,24 @@ void sweeps_tb32(swm_helm *h, float omega, int n) {
   }
 }
 
-// blocks of k_h_resid
-dim3 resid_grid(int nx, int ny) { return dim3((nx + RES_X - 1) / RES_X, (ny + RES_ROWS - 1) / RES_ROWS); }
+// rows of a column that a thread of k_h_resid walks: RES_ROWS, fewer where
+// that leaves the chip without eight blocks per SM (a row is a serial step of
+// 2 to 3 us; 256^2, FP32: 90 us with 32 rows, 9 with 2)
+int resid_rows(const swm_helm *h) {
+  int rows = RES_ROWS;
+  while (rows > 2 && (int64_t)((h->nx + RES_X - 1) / RES_X) * ((h->ny + rows - 1) / rows) < 8 * h->sms) rows /= 2;
+  return rows;
+}
+dim3 resid_grid(const swm_helm *h) {
+  const int rows = resid_rows(h);
+  return dim3((h->nx + RES_X - 1) / RES_X, (h->ny + rows - 1) / rows);
+}
 
 // ||rhs - A psi||^2 (FP64 accumulation); r written when wanted
 template <typename T>
 int resid2(swm_helm *h, const T *rhs, const T *psi, double *r, double *out) {
-  const dim3 g = resid_grid(h->nx, h->ny);
-  k_h_resid<T><<<g, RES_X, 0, h->stream>>>(h->nx, h->ny, h->cx, h->cy, h->cc, h->mask, rhs, psi, r, h->partial);
+  const dim3 g = resid_grid(h);
+  k_h_resid<T><<<g, RES_X, 0, h->stream>>>(h->nx, h->ny, resid_rows(h), h->cx, h->cy, h->cc, h->mask, rhs, psi, r, h->partial);
   k_h_final<<<1, 256, 0, h->stream>>>(h->partial, (int)(g.x * g.y), h->out);
   h->launches += 2;
   SWM_CK(cudaGetLastError());
@@ -601,7 +612,8 @@ int swm_helm_create(int nx, int ny, double dx, double dy, double lambda, const d
     hinv[k] = 1. / H[k];
     hinv32[k] = (float)hinv[k];
   }
-  const dim3 rg = resid_grid(nx, ny);
+  if (cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) h->sms = 1;
+  const dim3 rg = resid_grid(h);
   bool ok = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaMalloc((void **)&h->hinv, n * 8) == cudaSuccess && cudaMalloc((void **)&h->psi, n * 8) == cudaSuccess &&
             cudaMalloc((void **)&h->rhs, n * 8) == cudaSuccess && cudaMalloc((void **)&h->r, n * 8) == cudaSuccess &&
