@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include "ctx.h"
 
@@ -146,6 +147,22 @@ __global__ void __launch_bounds__(H64_T) k_h_sweep64(int nx, int ny, unsigned W,
   }
 }
 
+// the reciprocal diagonals of the tiled sweeps, by the expressions of k_h_sweep32
+__global__ void k_h_rcc32(int nx, int ny, const float *__restrict__ h, float rdx2, float rdy2, float lambda,
+                            const int8_t *__restrict__ mask, float *rcc) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= nx || j >= ny) return;
+  const size_t k = (size_t)i + (size_t)nx * j;
+  const float hk = h[k];
+  const float cxw = i > 0 ? face32(hk, h[k - 1], rdx2) : 0.f;
+  const float cxe = i < nx - 1 ? face32(h[k + 1], hk, rdx2) : 0.f;
+  const float cys = j > 0 ? face32(hk, h[k - nx], rdy2) : 0.f;
+  const float cyn = j < ny - 1 ? face32(h[k + nx], hk, rdy2) : 0.f;
+  const float d = 1.f / (-(((cxw + cxe) + cys) + cyn) - lambda);
+  // 0 stands for land; an ocean diagonal that overflowed gives NaN, as its update would
+  rcc[k] = mask[k] ? (d != 0.f ? d : NAN) : 0.f;
+}
+
 // one colour of an FP32 sweep over the whole grid (the arithmetic of k_h_tbr)
 __global__ void k_h_sweep32(int nx, int ny, const float *__restrict__ h, const int8_t *__restrict__ mask,
                             const float *__restrict__ rhs, float *psi, float rdx2, float rdy2, float lambda,
@@ -168,116 +185,243 @@ __global__ void k_h_sweep32(int nx, int ny, const float *__restrict__ h, const i
   psi[k] = sor32_update(psi[k], rhs[k], cxw, cxe, cys, cyn, rcc, w, e, s, n, omega);
 }
 
-// K red-black sweeps of FP32 SOR on a region of 64 columns by YM rows
-// (interior 64 - 4K by YM - 4K, halo 2K), each thread owning, for the whole
-// launch, the cell pair of region columns 2tx (cell a) and 2tx + 1 (cell b)
-// in rows ty + Ym.  A pair's face coefficients, reciprocal diagonals and rhs
-// are formed once per launch and kept in registers (the pair shares its
-// inner face).  psi is kept in shared memory split by column parity, so a
-// warp's accesses are contiguous, and each cell's inner neighbour is the
-// thread's own register.  Every neighbour of a cell has the other colour, so
-// a pass reads only what the previous passes wrote.  Halo cells are relaxed
-// with the arithmetic of the global sweep (sor32_update, same coefficients),
-// so after 2K passes the interior equals K global sweeps bit for bit; rows
-// that can no longer reach the interior are skipped.  Cells outside the grid
-// hold psi = 0 and are never relaxed.
-// TBR_Y x 32 threads per block, TBR_M rows per thread (64 registers: 2
-// blocks, 32 warps per SM); TBR_Y even, so a thread's cells a share one
-// colour
-constexpr int TBR_Y = 16, TBR_M = 3;
-template <int K>
-__global__ void __launch_bounds__(32 * TBR_Y, 2) k_h_tbr(int nx, int ny, const float *__restrict__ hin,
-                                                  const int8_t *__restrict__ mask, const float *__restrict__ rhs,
-                                                  const float *__restrict__ pin, float *__restrict__ pout, float rdx2,
-                                                  float rdy2, float lambda, float omega) {
-  constexpr int M = TBR_M, Y = TBR_Y, W = 2 * K, RY = Y * M, TX = 64 - 2 * W, TY = RY - 2 * W;
-  __shared__ float sa[RY][32], sb[RY][32];  // psi of the even / odd region columns
-  __shared__ float ha[RY][32], hb[RY][32];  // 1/H, read while forming the coefficients
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x0 = blockIdx.x * TX - W, y0 = blockIdx.y * TY - W;
-  const int gxa = x0 + 2 * tx, gxb = gxa + 1;
-  float pa[M], pb[M], ra[M], rb[M];                       // psi and rhs of cells a and b
-  float cwa[M], cm[M], ceb[M], csa[M], cna[M], csb[M], cnb[M];  // face coefficients (cm: a's east = b's west)
-  float qa[M], qb[M];                                     // reciprocal diagonals
-  unsigned relax = 0;                                     // bit 2m: cell a of row m is relaxed, 2m + 1: cell b
+// The update of two cells of a colour at once, in packed FP32x2 instructions
+// (each half rounded as sor32_update rounds it; a - b as a + (-1) b, exact)
+__device__ __forceinline__ float2 sor32_update2(float2 p, float2 r, float2 cxw, float2 cxe, float2 cys, float2 cyn,
+                                                float2 rcc, float2 w, float2 e, float2 s, float2 n, float omega) {
+  const float2 neg = make_float2(-1.f, -1.f);
+  const float2 off = __ffma2_rn(cyn, n, __ffma2_rn(cys, s, __ffma2_rn(cxe, e, __fmul2_rn(cxw, w))));
+  const float2 gs = __fmul2_rn(__ffma2_rn(off, neg, r), rcc);
+  return __ffma2_rn(make_float2(omega, omega), __ffma2_rn(p, neg, gs), p);
+}
+
+// K red-black sweeps of FP32 SOR on a region of 64 columns by 96 rows (48 rows
+// on small grids), of which the interior, 2K cells from its edge, is written.
+// A thread owns, for the whole region, four cells a0 b0 a1 b1 of adjacent
+// columns in each of TBR_M rows; a0 and a1 (b0 and b1) have one colour and are
+// updated together.  Their face coefficients, reciprocal diagonals and rhs are
+// kept in registers.  psi is kept in shared memory by column parity, so that a
+// pair's neighbours to the north and south are one 64-bit load each; to the
+// east and west they are the thread's own registers and one shuffle.  The
+// half-warps of warp w of NW own rows w + NW h + 2 NW m (h the half, m < TBR_M),
+// which have one parity as NW is even, so a pass is one warp-uniform branch.
+// Every neighbour of a cell has the other colour, so a pass reads only what
+// the previous passes wrote.  Halo cells are relaxed with the arithmetic of
+// the global sweep (same coefficients), so after 2K passes the interior equals
+// K global sweeps bit for bit; what the passes leave in cells that no longer
+// reach the interior is not used.  Cells outside the grid hold psi = 0 and are
+// never relaxed, nor is the region's outer ring (its neighbours lie outside).
+//
+// What a launch of 4 sweeps of 4096^2 took: 177 us with two columns of a
+// thread relaxed one by one, coefficients formed and divided for in each
+// launch; as much with packed pairs and four fields read instead, of which
+// 105 us before the first pass; 163 us with the next region's fields fetched
+// during the passes (k_h_tbr_stream); 149 us with 96 rows instead of 48 (the
+// passes and the loads repeat 1.6 cells per written cell, not 2); 136 us with
+// faces formed from the reciprocal depth (four fields read, not five).  The
+// passes themselves take about 60 us, the four fields and the result 50 us of
+// HBM.  80 registers: 24 warps per SM, in one block or two.
+constexpr int TBR_M = 2;
+constexpr int tbr_rows(int nw) { return 2 * nw * TBR_M; }  // rows of a block of nw warps
+struct Region32 {  // what the tiled sweeps read: reciprocal depth, reciprocal diagonal (0 on land)
+  int nx, ny;
+  float rdx2, rdy2;
+  const float *hinv, *rcc;
+};
+
+// the cells of one thread: psi, rhs, reciprocal diagonal of (a0, a1) and (b0,
+// b1), and their faces
+struct TbrCells {
+  float2 p[2][TBR_M], f[2][TBR_M], q[2][TBR_M];
+  float2 cw[TBR_M], cm[TBR_M], ce[TBR_M];  // (a0 west, a1 west), (a0 east, a1 east), (b0 east, b1 east)
+  float2 cs[2][TBR_M], cn[2][TBR_M];
+  unsigned relax = 0;  // bit 4m + c: cell c of row m is relaxed
+
+  // row m from the four columns' values; h, hs, hn: reciprocal depth of this
+  // row, the row to its south and the row to its north; (gx, gy): the first
+  // column's cell in the grid, edge: the region reaches the grid's edge, where
+  // faces are 0.  The faces of the ring, which need cells outside the region,
+  // are not used.
+  __device__ __forceinline__ void set(int m, int ly, int rows, int tx, const Region32 &g, int gx, int gy, bool edge,
+                                      const float *pv, const float *fv, const float *h, const float *hs,
+                                      const float *hn, const float *d) {
+    unsigned mk = 0;
 #pragma unroll
-  for (int m = 0; m < M; m++) {
-    const int ly = ty + Y * m, gy = y0 + ly;
-    const bool iny = gy >= 0 && gy < ny;
-    const bool ina = iny && gxa >= 0 && gxa < nx, inb = iny && gxb >= 0 && gxb < nx;
-    const size_t ka = ina ? (size_t)gxa + (size_t)nx * gy : 0, kb = inb ? (size_t)gxb + (size_t)nx * gy : 0;
-    pa[m] = ina ? pin[ka] : 0.f;
-    pb[m] = inb ? pin[kb] : 0.f;
-    ra[m] = ina ? rhs[ka] : 0.f;
-    rb[m] = inb ? rhs[kb] : 0.f;
-    ha[ly][tx] = ina ? hin[ka] : 1.f;
-    hb[ly][tx] = inb ? hin[kb] : 1.f;
-    sa[ly][tx] = pa[m];
-    sb[ly][tx] = pb[m];
-    // the region's outer ring is never relaxed (its neighbours lie outside)
-    const bool inner = ly >= 1 && ly < RY - 1;
-    if (inner && ina && tx > 0 && mask[ka]) relax |= 1u << (2 * m);
-    if (inner && inb && tx < 31 && mask[kb]) relax |= 2u << (2 * m);
-  }
-  __syncthreads();
+    for (int c = 0; c < 4; c++) mk |= d[c] != 0.f ? 1u << c : 0u;
+    if (ly == 0 || ly == rows - 1) mk = 0;  // the ring
+    if (tx == 0) mk &= ~1u;
+    if (tx == 15) mk &= ~8u;
+    relax |= mk << (4 * m);
+    float x[4], ys[4], yn[4];
+    x[0] = face32(h[0], __shfl_up_sync(0xffffffffu, h[3], 1, 16), g.rdx2);
 #pragma unroll
-  for (int m = 0; m < M; m++) {
-    const int ly = ty + Y * m, gy = y0 + ly;
-    cwa[m] = cm[m] = ceb[m] = csa[m] = cna[m] = csb[m] = cnb[m] = qa[m] = qb[m] = 0.f;
-    const bool da = (relax >> (2 * m)) & 1, db = (relax >> (2 * m + 1)) & 1;
-    const float hka = ha[ly][tx], hkb = hb[ly][tx];
-    if (da || db) cm[m] = gxa < nx - 1 && gxb > 0 ? face32(hkb, hka, rdx2) : 0.f;
-    if (da) {
-      cwa[m] = gxa > 0 ? face32(hka, hb[ly][tx - 1], rdx2) : 0.f;
-      csa[m] = gy > 0 ? face32(hka, ha[ly - 1][tx], rdy2) : 0.f;
-      cna[m] = gy < ny - 1 ? face32(ha[ly + 1][tx], hka, rdy2) : 0.f;
-      qa[m] = 1.f / (-(((cwa[m] + cm[m]) + csa[m]) + cna[m]) - lambda);
+    for (int c = 0; c < 4; c++) {
+      if (c) x[c] = face32(h[c], h[c - 1], g.rdx2);
+      ys[c] = face32(h[c], hs[c], g.rdy2);
+      yn[c] = face32(hn[c], h[c], g.rdy2);
     }
-    if (db) {
-      ceb[m] = gxb < nx - 1 ? face32(ha[ly][tx + 1], hkb, rdx2) : 0.f;
-      csb[m] = gy > 0 ? face32(hkb, hb[ly - 1][tx], rdy2) : 0.f;
-      cnb[m] = gy < ny - 1 ? face32(hb[ly + 1][tx], hkb, rdy2) : 0.f;
-      qb[m] = 1.f / (-(((cm[m] + ceb[m]) + csb[m]) + cnb[m]) - lambda);
-    }
-  }
-  // colour of this thread's cells a ((gx + gy) & 1, the same in all its rows)
-  const int ca = (x0 + y0 + ty) & 1;
-  // flat views: the ring columns' outer neighbours (never used: those cells
-  // are not relaxed) then stay inside the arrays
-  const float *fa = &sa[0][0], *fb = &sb[0][0];
+    if (edge) {
 #pragma unroll
-  for (int pass = 0; pass < 2 * K; pass++) {
-    const int lo = pass + 1, hi = RY - pass - 1;  // rows that still reach the interior
-    const bool do_a = ca == (pass & 1);           // warp-uniform
-#pragma unroll
-    for (int m = 0; m < M; m++) {
-      const int ly = ty + Y * m, l = ly * 32 + tx;
-      // rows Ym .. Ym + Y - 1 lie in [lo, hi) in every pass unless m is the
-      // first or last row group: only those test the row (warp-uniform)
-      const bool mid = Y * m >= 2 * K && Y * m + Y <= RY - 2 * K;
-      if (!mid && (ly < lo || ly >= hi)) continue;
-      // relaxed as in the global sweep; cells not relaxed (land, outside the
-      // grid, the region's ring) store their value back unchanged
-      if (do_a) {
-        const float v = sor32_update(pa[m], ra[m], cwa[m], cm[m], csa[m], cna[m], qa[m], fb[l - 1], pb[m],
-                                     fa[l - 32], fa[l + 32], omega);
-        pa[m] = ((relax >> (2 * m)) & 1) ? v : pa[m];
-        sa[ly][tx] = pa[m];
-      } else {
-        const float v = sor32_update(pb[m], rb[m], cm[m], ceb[m], csb[m], cnb[m], qb[m], pa[m], fa[l + 1],
-                                     fb[l - 32], fb[l + 32], omega);
-        pb[m] = ((relax >> (2 * m + 1)) & 1) ? v : pb[m];
-        sb[ly][tx] = pb[m];
+      for (int c = 0; c < 4; c++) {
+        if (gx + c <= 0 || gx + c >= g.nx) x[c] = 0.f;
+        if (gy <= 0) ys[c] = 0.f;
+        if (gy >= g.ny - 1) yn[c] = 0.f;
       }
     }
+    const float xe = __shfl_down_sync(0xffffffffu, x[0], 1, 16);  // the next thread's first column (b1's east face)
+    cw[m] = make_float2(x[0], x[2]);
+    cm[m] = make_float2(x[1], x[3]);
+    ce[m] = make_float2(x[2], xe);
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      p[c][m] = make_float2(pv[c], pv[c + 2]);
+      f[c][m] = make_float2(fv[c], fv[c + 2]);
+      q[c][m] = make_float2(d[c], d[c + 2]);
+      cs[c][m] = make_float2(ys[c], ys[c + 2]);
+      cn[c][m] = make_float2(yn[c], yn[c + 2]);
+    }
+  }
+};
+
+// the passes of one launch; sp: psi of the even / odd region columns, a pair
+// per thread; ca: colour of the thread's cells a ((gx + gy) & 1, one in all its rows)
+template <int K, int NW>
+__device__ __forceinline__ void tbr_passes(TbrCells &t, float2 (*sp)[tbr_rows(NW)][16], int tx, int r0, int ca,
+                                           float omega) {
+  constexpr int M = TBR_M, RY = tbr_rows(NW);
+  auto pass = [&](auto which) {  // 0: cells a, 1: cells b
+    constexpr int c = decltype(which)::value;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      const int ly = r0 + 2 * NW * m;
+      // (the ring rows' loads stay inside the arrays)
+      const float2 s = sp[c][m ? ly - 1 : max(ly - 1, 0)][tx], n = sp[c][m == M - 1 ? min(ly + 1, RY - 1) : ly + 1][tx];
+      float2 v;
+      if (c == 0) {
+        const float w = __shfl_up_sync(0xffffffffu, t.p[1][m].y, 1, 16);
+        v = sor32_update2(t.p[0][m], t.f[0][m], t.cw[m], t.cm[m], t.cs[0][m], t.cn[0][m], t.q[0][m],
+                          make_float2(w, t.p[1][m].x), t.p[1][m], s, n, omega);
+      } else {
+        const float e = __shfl_down_sync(0xffffffffu, t.p[0][m].x, 1, 16);
+        v = sor32_update2(t.p[1][m], t.f[1][m], t.cm[m], t.ce[m], t.cs[1][m], t.cn[1][m], t.q[1][m], t.p[0][m],
+                          make_float2(t.p[0][m].y, e), s, n, omega);
+      }
+      // cells not relaxed (land, outside the grid, the ring) keep their value
+      t.p[c][m].x = (t.relax >> (4 * m + c)) & 1 ? v.x : t.p[c][m].x;
+      t.p[c][m].y = (t.relax >> (4 * m + c + 2)) & 1 ? v.y : t.p[c][m].y;
+      sp[c][ly][tx] = t.p[c][m];
+    }
+  };
+#pragma unroll
+  for (int k = 0; k < 2 * K; k++) {
+    if (ca == (k & 1)) pass(std::integral_constant<int, 0>{});  // warp-uniform
+    else pass(std::integral_constant<int, 1>{});
     __syncthreads();
   }
+}
+
+// any grid: a block per region, values read as the thread needs them
+template <int K, int NW>
+__global__ void __launch_bounds__(32 * NW, 24 / NW) k_h_tbr(Region32 co, const float *__restrict__ rhs, const float *__restrict__ pin,
+                                                             float *__restrict__ pout, float omega) {
+  const int nx = co.nx, ny = co.ny;
+  constexpr int M = TBR_M, W = 2 * K, RY = tbr_rows(NW), TX = 64 - 2 * W, TY = RY - 2 * W;
+  __shared__ float2 sp[2][RY][16];
+  const int tx = threadIdx.x & 15, r0 = (threadIdx.x >> 5) + NW * ((threadIdx.x >> 4) & 1);
+  const int x0 = blockIdx.x * TX - W, y0 = blockIdx.y * TY - W, gx = x0 + 4 * tx;
+  TbrCells t;
 #pragma unroll
   for (int m = 0; m < M; m++) {
-    const int ly = ty + Y * m, gy = y0 + ly;
+    const int ly = r0 + 2 * NW * m, gy = y0 + ly;
+    auto load = [&](const float *a, int g, float *v) {
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        v[c] = g >= 0 && g < ny && gx + c >= 0 && gx + c < nx ? a[(size_t)(gx + c) + (size_t)nx * g] : 0.f;
+    };
+    float pv[4], fv[4], h[4], hs[4], hn[4], d[4];
+    load(pin, gy, pv);
+    load(rhs, gy, fv);
+    load(co.hinv, gy, h);
+    load(co.hinv, gy - 1, hs);
+    load(co.hinv, gy + 1, hn);
+    load(co.rcc, gy, d);
+    t.set(m, ly, RY, tx, co, gx, gy, true, pv, fv, h, hs, hn, d);
+    for (int c = 0; c < 2; c++) sp[c][ly][tx] = t.p[c][m];
+  }
+  __syncthreads();
+  tbr_passes<K, NW>(t, sp, tx, r0, (x0 + y0 + r0) & 1, omega);
+#pragma unroll
+  for (int m = 0; m < M; m++) {
+    const int ly = r0 + 2 * NW * m, gy = y0 + ly;
     if (ly < W || ly >= RY - W || gy >= ny) continue;
-    if (2 * tx >= W && 2 * tx < 64 - W && gxa < nx) pout[(size_t)gxa + (size_t)nx * gy] = pa[m];
-    if (2 * tx + 1 >= W && 2 * tx + 1 < 64 - W && gxb < nx) pout[(size_t)gxb + (size_t)nx * gy] = pb[m];
+    const float v[4] = {t.p[0][m].x, t.p[1][m].x, t.p[0][m].y, t.p[1][m].y};
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      if (4 * tx + c >= W && 4 * tx + c < 64 - W && gx + c < nx) pout[(size_t)(gx + c) + (size_t)nx * gy] = v[c];
+  }
+}
+
+// Where rows and regions start at multiples of four columns (nx and 2K are
+// multiples of 4): persistent blocks take region after region, and while one
+// is relaxed the next one's four fields come into shared memory by
+// asynchronous 16-byte copies.  3 sweeps of 4096^2 and rows of odd length
+// stay with k_h_tbr, which can start at any column (4095^2: 168 us for 4).
+constexpr int TBR_FIELDS = 4;
+template <int K, int NW>
+__global__ void __launch_bounds__(32 * NW, 24 / NW) k_h_tbr_stream(int nbx, int tiles, Region32 co,
+                                                                    const float *__restrict__ rhs,
+                                                                    const float *__restrict__ pin,
+                                                                    float *__restrict__ pout, float omega) {
+  const int nx = co.nx, ny = co.ny;
+  constexpr int M = TBR_M, W = 2 * K, RY = tbr_rows(NW), TX = 64 - 2 * W, TY = RY - 2 * W;
+  static_assert(W % 4 == 0, "regions start at multiples of four columns");
+  extern __shared__ float4 stage[];  // [field][row][16]: psi, rhs, hinv, rcc
+  __shared__ float2 sp[2][RY][16];
+  const int tx = threadIdx.x & 15, r0 = (threadIdx.x >> 5) + NW * ((threadIdx.x >> 4) & 1);
+  const float *src[TBR_FIELDS] = {pin, rhs, co.hinv, co.rcc};
+  auto fetch = [&](int tile) {
+    const int x0 = (tile % nbx) * TX - W, y0 = (tile / nbx) * TY - W;
+    for (int e = threadIdx.x; e < RY * 16; e += 32 * NW) {
+      const int ly = e >> 4, gx = x0 + 4 * (e & 15), gy = y0 + ly;
+      const bool in = gy >= 0 && gy < ny && gx >= 0 && gx < nx;
+      const size_t k = in ? (size_t)gx + (size_t)nx * gy : 0;
+#pragma unroll
+      for (int f = 0; f < TBR_FIELDS; f++) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage + f * RY * 16 + e);
+        // outside the grid no byte is read and zeros are written
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src[f] + k), "r"(in ? 16 : 0) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if ((int)blockIdx.x < tiles) fetch(blockIdx.x);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int x0 = (tile % nbx) * TX - W, y0 = (tile / nbx) * TY - W, gx = x0 + 4 * tx;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const bool edge = x0 <= 0 || y0 <= 0 || x0 + 64 >= nx || y0 + RY >= ny;
+    TbrCells t;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      const int ly = r0 + 2 * NW * m, e = ly * 16 + tx;
+      const float4 a = stage[e], b = stage[RY * 16 + e], c = stage[2 * RY * 16 + e], d = stage[3 * RY * 16 + e],
+                   s = stage[2 * RY * 16 + (m ? e - 16 : max(e - 16, tx))],
+                   n = stage[2 * RY * 16 + (m == M - 1 ? min(ly + 1, RY - 1) * 16 + tx : e + 16)];
+      const float pv[4] = {a.x, a.y, a.z, a.w}, fv[4] = {b.x, b.y, b.z, b.w}, h[4] = {c.x, c.y, c.z, c.w},
+                  dv[4] = {d.x, d.y, d.z, d.w}, hs[4] = {s.x, s.y, s.z, s.w}, hn[4] = {n.x, n.y, n.z, n.w};
+      t.set(m, ly, RY, tx, co, gx, y0 + ly, edge, pv, fv, h, hs, hn, dv);
+      for (int q = 0; q < 2; q++) sp[q][ly][tx] = t.p[q][m];
+    }
+    __syncthreads();
+    if (tile + (int)gridDim.x < tiles) fetch(tile + gridDim.x);
+    tbr_passes<K, NW>(t, sp, tx, r0, (x0 + y0 + r0) & 1, omega);
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      const int ly = r0 + 2 * NW * m, gy = y0 + ly;
+      if (ly >= W && ly < RY - W && gy < ny && 4 * tx >= W && 4 * tx < 64 - W && gx < nx)
+        *reinterpret_cast<float4 *>(pout + (size_t)gx + (size_t)nx * gy) =
+            make_float4(t.p[0][m].x, t.p[1][m].x, t.p[0][m].y, t.p[1][m].y);
+    }
   }
 }
 
@@ -410,9 +554,11 @@ struct swm_helm {
   cudaStream_t stream = nullptr;
   double *hinv = nullptr, *psi = nullptr, *rhs = nullptr, *r = nullptr, *partial = nullptr, *out = nullptr;
   double *host = nullptr;  // pinned, 1 double
+  float *rcc32 = nullptr;  // reciprocal diagonals of the tiled FP32 sweeps
   float *hinv32 = nullptr, *e32 = nullptr, *r32 = nullptr, *e32b = nullptr;  // e32b: ping-pong of e32
   int tbk = 4;  // sweeps per temporally blocked FP32 launch
   int sms = 0;
+  int tb_blocks[2][2] = {};  // resident blocks of the streamed launches: 2 and 4 sweeps, 12 and 24 warps (0: not asked yet)
   int8_t *mask = nullptr;
   dim3 blk = dim3(64, 4);
   int64_t launches = 0;
@@ -480,13 +626,40 @@ void sweep32(swm_helm *h, float omega, dim3 b) {
   h->launches += 2;
 }
 
+template <int K, int NW>
+int launch_tb32(swm_helm *h, float omega) {
+  constexpr int TX = 64 - 4 * K, TY = tbr_rows(NW) - 4 * K;
+  const dim3 g((h->nx + TX - 1) / TX, (h->ny + TY - 1) / TY), b(32 * NW);
+  const Region32 co = {h->nx, h->ny, (float)(1. / (h->dx * h->dx)), (float)(1. / (h->dy * h->dy)), h->hinv32, h->rcc32};
+  if constexpr (K % 2 == 0) {
+    if (h->nx % 4 == 0) {
+      constexpr int bytes = TBR_FIELDS * tbr_rows(NW) * 16 * (int)sizeof(float4);
+      int &blocks = h->tb_blocks[K / 2 - 1][NW == 24];
+      if (blocks == 0) {
+        int per_sm = 0;
+        SWM_CK(cudaFuncSetAttribute(k_h_tbr_stream<K, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        SWM_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_h_tbr_stream<K, NW>, 32 * NW, bytes));
+        blocks = std::max(1, per_sm) * h->sms;
+      }
+      const int tiles = (int)(g.x * g.y);
+      k_h_tbr_stream<K, NW><<<std::min(tiles, blocks), b, bytes, h->stream>>>((int)g.x, tiles, co, h->r32, h->e32,
+                                                                              h->e32b, omega);
+      SWM_CK(cudaGetLastError());
+      return SWM_GPU_OK;
+    }
+  }
+  k_h_tbr<K, NW><<<g, b, 0, h->stream>>>(co, h->r32, h->e32, h->e32b, omega);
+  SWM_CK(cudaGetLastError());
+  return SWM_GPU_OK;
+}
+
+// Blocks of 24 warps where every SM gets one of their regions, else blocks of
+// 12 with half the rows: 256^2 5.9 against 7.8 us, 768^2 (160 tall regions)
+// and above faster with 24.
 template <int K>
-void launch_tb32(swm_helm *h, float omega) {
-  constexpr int TX = 64 - 4 * K, TY = TBR_Y * TBR_M - 4 * K;
-  const dim3 g((h->nx + TX - 1) / TX, (h->ny + TY - 1) / TY), b(32, TBR_Y);
-  const float rdx2 = (float)(1. / (h->dx * h->dx)), rdy2 = (float)(1. / (h->dy * h->dy)), lam = (float)h->lambda;
-  k_h_tbr<K><<<g, b, 0, h->stream>>>(h->nx, h->ny, h->hinv32, h->mask, h->r32, h->e32, h->e32b, rdx2, rdy2, lam,
-                                     omega);
+int launch_tb32(swm_helm *h, float omega) {
+  const int nx = (h->nx + 63 - 4 * K) / (64 - 4 * K), ny = (h->ny + 95 - 4 * K) / (96 - 4 * K);
+  return (int64_t)nx * ny >= h->sms ? launch_tb32<K, 24>(h, omega) : launch_tb32<K, 12>(h, omega);
 }
 
 // whole temporally blocked launches in n sweeps (none when tbk is 0: global
@@ -495,15 +668,16 @@ int tb_part(const swm_helm *h, int n) { return h->tbk > 0 ? n - n % h->tbk : 0; 
 
 // n FP32 sweeps (a multiple of h->tbk) on A e = r32, ping-ponging e32/e32b;
 // the result ends in h->e32
-void sweeps_tb32(swm_helm *h, float omega, int n) {
+int sweeps_tb32(swm_helm *h, float omega, int n) {
   for (int s = 0; s < n && h->tbk > 0; s += h->tbk) {
-    if (h->tbk == 4) launch_tb32<4>(h, omega);
-    else if (h->tbk == 3) launch_tb32<3>(h, omega);
-    else if (h->tbk == 2) launch_tb32<2>(h, omega);
-    else launch_tb32<1>(h, omega);
+    if (h->tbk == 4) HTRY(launch_tb32<4>(h, omega));
+    else if (h->tbk == 3) HTRY(launch_tb32<3>(h, omega));
+    else if (h->tbk == 2) HTRY(launch_tb32<2>(h, omega));
+    else HTRY(launch_tb32<1>(h, omega));
     std::swap(h->e32, h->e32b);
     h->launches++;
   }
+  return SWM_GPU_OK;
 }
 
 // rows of a column that a thread of k_h_resid walks: RES_ROWS, fewer where
@@ -560,7 +734,7 @@ int inner32(swm_helm *h, float omega, double tol, int max_sweeps, int *sweeps, d
     // 2 * HELM_CHECK sweeps between checks of the correction equation
     int blk = std::min(2 * HELM_CHECK, max_sweeps - s);
     const int tb = tb_part(h, blk);
-    sweeps_tb32(h, omega, tb);
+    HTRY(sweeps_tb32(h, omega, tb));
     for (int q = tb; q < blk; q++) sweep32(h, omega, h->blk);
     s += blk;
     double e2 = 0.;
@@ -580,6 +754,7 @@ void helm_free(swm_helm *h) {
   cudaFree(h->hinv); cudaFree(h->psi); cudaFree(h->rhs); cudaFree(h->r); cudaFree(h->partial); cudaFree(h->out);
   cudaFreeHost(h->host);
   cudaFree(h->hinv32); cudaFree(h->e32); cudaFree(h->r32); cudaFree(h->mask); cudaFree(h->e32b);
+  cudaFree(h->rcc32);
   cudaFree(h->cx); cudaFree(h->cy); cudaFree(h->cc); cudaFree(h->rcc);
   for (int col = 0; col < 2; col++) {
     for (int f = 0; f < 4; f++) cudaFree(h->s64.c[col][f]);
@@ -622,6 +797,7 @@ int swm_helm_create(int nx, int ny, double dx, double dy, double lambda, const d
             cudaMalloc((void **)&h->hinv32, n * 4) == cudaSuccess && cudaMalloc((void **)&h->e32, n * 4) == cudaSuccess &&
             cudaMalloc((void **)&h->r32, n * 4) == cudaSuccess && cudaMalloc((void **)&h->mask, n) == cudaSuccess &&
             cudaMalloc((void **)&h->e32b, n * 4) == cudaSuccess &&
+            cudaMalloc((void **)&h->rcc32, n * 4) == cudaSuccess &&
             cudaMalloc((void **)&h->cx, n * 8) == cudaSuccess && cudaMalloc((void **)&h->cy, n * 8) == cudaSuccess &&
             cudaMalloc((void **)&h->cc, n * 8) == cudaSuccess && cudaMalloc((void **)&h->rcc, n * 8) == cudaSuccess;
   if (!ok) {
@@ -634,7 +810,9 @@ int swm_helm_create(int nx, int ny, double dx, double dy, double lambda, const d
   SWM_CK(cudaMemcpyAsync(h->mask, ocean, n, cudaMemcpyHostToDevice, h->stream));
   dim3 b(32, 8), g((nx + 31) / 32, (ny + 7) / 8);
   k_h_coeff64<<<g, b, 0, h->stream>>>(nx, ny, h->hinv, 1. / (dx * dx), 1. / (dy * dy), lambda, h->cx, h->cy, h->cc, h->rcc);
-  h->launches++;
+  k_h_rcc32<<<g, b, 0, h->stream>>>(nx, ny, h->hinv32, (float)(1. / (dx * dx)), (float)(1. / (dy * dy)),
+                                    (float)lambda, h->mask, h->rcc32);
+  h->launches += 2;
   SWM_CK(cudaGetLastError());
   SWM_CK(cudaStreamSynchronize(h->stream));
   *out = h;
@@ -783,9 +961,9 @@ int swm_helm_autotune(swm_helm *h, const double *rhs, double omega_lo, double om
     float kbest = 1e30f;
     for (int kk : {1, 2, 3, 4}) {
       h->tbk = kk;
-      sweeps_tb32(h, 1.f, 4);
+      HTRY(sweeps_tb32(h, 1.f, 4));
       SWM_CK(cudaEventRecord(a, h->stream));
-      sweeps_tb32(h, 1.f, 8);
+      HTRY(sweeps_tb32(h, 1.f, 8));
       SWM_CK(cudaEventRecord(b, h->stream));
       SWM_CK(cudaEventSynchronize(b));
       float ms;
@@ -803,7 +981,7 @@ int swm_helm_autotune(swm_helm *h, const double *rhs, double omega_lo, double om
     k_h_to32<<<nb, 256, 0, h->stream>>>(h->rhs, h->r32, h->e32, h->n, bn > 0 ? 1. / bn : 1.);
     h->launches++;
     const int tb = tb_part(h, trial_sweeps);
-    sweeps_tb32(h, (float)om, tb);
+    HTRY(sweeps_tb32(h, (float)om, tb));
     for (int s = tb; s < trial_sweeps; s++) sweep32(h, (float)om, h->blk);
     double e2;
     HTRY(resid2<float>(h, h->r32, h->e32, nullptr, &e2));
