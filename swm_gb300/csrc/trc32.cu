@@ -1,4 +1,4 @@
-// trc32.cu -- passive tracers on the FP32 compensated path, up to two tracers
+// trc32.cu -- passive tracers on the FP32 compensated path, up to four tracers
 // of a basin per launch.
 //
 // Formulas: TRC_tracer_incr (tracer_module.f90:154-209), TRC_initCoeffs
@@ -16,14 +16,13 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
-#include <type_traits>
 #include <vector>
 #include "ctx.h"
 #include "fused32.h"
 
 namespace swm {
 
-constexpr int TRC32_MAX = 2;  // tracers per launch (more run in several launches)
+constexpr int TRC32_MAX = 4;  // tracers per launch (more run in several launches)
 enum { RT_RDL, RT_RDT, RT_CV, RT_D8, RT_D10, RT_NR };
 
 struct Tracer32 {
@@ -51,11 +50,12 @@ __device__ __forceinline__ int wr(int a, int n) { return a < 0 ? a + n : (a >= n
 // 1 / thickness, 0 on dry land (C = CH * rD then takes the 0/0 there as 0)
 __device__ __forceinline__ float rthick(float d) { return d != 0.f ? __frcp_rn(d) : 0.f; }
 
-// One tracer's values (float) or two tracers' (float2): the arithmetic of two
-// runs in packed FP32x2 instructions, each half rounded as the scalar one, so
-// a tracer's results do not depend on how many share its launch.  Every
-// operation below is explicit, with the products that the compiler fused into
-// the sums of the scalar form fused here: results are that form's bit for bit.
+// One tracer's values (float), two tracers' (float2) or more (More, below): the
+// arithmetic of two runs in packed FP32x2 instructions, each half rounded as
+// the scalar one, so a tracer's results do not depend on how many share its
+// launch.  Every operation below is explicit, with the products that the
+// compiler fused into the sums of the scalar form fused here: results are that
+// form's bit for bit.
 __device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -82,14 +82,53 @@ __device__ __forceinline__ float2 vup(float2 v) { return make_float2(vup(v.x), v
 __device__ __forceinline__ float vdown(float v, int n) { return __shfl_down_sync(FULLM, v, n); }
 __device__ __forceinline__ float2 vdown(float2 v, int n) { return make_float2(vdown(v.x, n), vdown(v.y, n)); }
 
+// Three or four tracers: a pair and one more, or two pairs
+template <typename B>
+struct More {
+  float2 a;
+  B b;
+};
+template <typename B>
+__device__ __forceinline__ More<B> vadd(More<B> x, More<B> y) { return {vadd(x.a, y.a), vadd(x.b, y.b)}; }
+template <typename B>
+__device__ __forceinline__ More<B> vmul(More<B> x, More<B> y) { return {vmul(x.a, y.a), vmul(x.b, y.b)}; }
+template <typename B>
+__device__ __forceinline__ More<B> vfma(More<B> x, More<B> y, More<B> z) { return {vfma(x.a, y.a, z.a), vfma(x.b, y.b, z.b)}; }
+template <typename B>
+__device__ __forceinline__ More<B> vsub(More<B> x, More<B> y) { return {vsub(x.a, y.a), vsub(x.b, y.b)}; }
+template <typename B>
+__device__ __forceinline__ More<B> vsel(bool c, More<B> x, More<B> y) { return {vsel(c, x.a, y.a), vsel(c, x.b, y.b)}; }
+template <typename B>
+__device__ __forceinline__ More<B> vup(More<B> v) { return {vup(v.a), vup(v.b)}; }
+template <typename B>
+__device__ __forceinline__ More<B> vdown(More<B> v, int n) { return {vdown(v.a, n), vdown(v.b, n)}; }
+template <typename B>
+__device__ __forceinline__ float &half(More<B> &v, int q) { return q < 2 ? half(v.a, q) : half(v.b, q - 2); }
+template <>
+__device__ __forceinline__ More<float> vb<More<float>>(float s) { return {make_float2(s, s), s}; }
+template <>
+__device__ __forceinline__ More<float2> vb<More<float2>>(float s) { return {make_float2(s, s), make_float2(s, s)}; }
+template <int NT>
+struct Values;
+template <>
+struct Values<1> { using type = float; };
+template <>
+struct Values<2> { using type = float2; };
+template <>
+struct Values<3> { using type = More<float>; };
+template <>
+struct Values<4> { using type = More<float2>; };
+
 // Advective flux of CH through the face between L and R (R east or north of
 // L, Lm behind L, Rp beyond R) for the velocity vel (times the row's cosine at
-// a north face): the third-order upwind-biased value (-1, 5, 2)/6 from the
-// upwind side where all four cells are ocean (FLUX 1), the mask-weighted mean
-// elsewhere.  FAST: all masks are 1.
+// a north face; 0, or NaN where it is not finite, at a closed face): the
+// third-order upwind-biased value (-1, 5, 2)/6 from the upwind side where all
+// four cells are ocean (FLUX 1), the mask-weighted mean elsewhere.  FAST: all
+// masks are 1.  The mean's halves are taken before the sum: where a field
+// overflows, which cells hold infinities and NaNs does not depend on the body.
 template <bool FAST, int FLUX, typename V>
-__device__ __forceinline__ V face_flux(float vel, V cLm, V cL, V cR, V cRp, unsigned open, unsigned oLm, unsigned oL,
-                                       unsigned oR, unsigned oRp) {
+__device__ __forceinline__ V face_flux(float vel, V cLm, V cL, V cR, V cRp, unsigned oLm, unsigned oL, unsigned oR,
+                                       unsigned oRp) {
   V f;
   if (FLUX == 1) {
     const bool pos = vel >= 0.f;
@@ -98,12 +137,12 @@ __device__ __forceinline__ V face_flux(float vel, V cLm, V cL, V cR, V cRp, unsi
     f = vmul(vmul(t, vb<V>(1.f / 6.f)), vb<V>(vel));
     if (FAST) return f;
   }
-  if (FAST) return vmul(vadd(cL, cR), vb<V>(0.5f * vel));
-  const unsigned den = oL + oR;
   const V zero = vb<V>(0.f);
-  const V mean = vmul(vadd(vsel(oL, cL, zero), vsel(oR, cR, zero)), vb<V>(den == 2 ? 0.5f * vel : vel));
-  if (FLUX == 1 && (oLm & oL & oR & oRp)) return vsel(open, f, zero);
-  return vsel(open && den, mean, zero);
+  const V hf = vb<V>(FAST || (oL & oR) ? 0.5f : 1.f);
+  const V a = FAST ? cL : vsel(oL, cL, zero), b = FAST ? cR : vsel(oR, cR, zero);
+  const V mean = vmul(vfma(a, hf, vmul(b, hf)), vb<V>(vel));
+  if (FLUX == 1 && (oLm & oL & oR & oRp)) return f;
+  return mean;
 }
 
 // (hi + lo + inc) * (1 - dp) as a new (hi, lo) pair, inc = dt x (not rounded
@@ -129,18 +168,21 @@ __device__ __forceinline__ void comp_update(V hi, V lo, V dt, V x, bool decay, V
 // the strip keeping the last rows of CH (hi + lo), thickness and masks in
 // registers, and updates row J-2 once row J is in.
 // Issue-bound: where the whole window of a warp is ocean (a warp vote) a body
-// with every mask test folded away runs, and two tracers share packed
-// instructions.  2049^2, two tracers, upwind-biased: 117 us a step with the mask
-// tests and two scalar tracers, 89 now; 2.83 -> 3.66 TB/s of the 78 B a point.
+// with every mask test folded away runs, and tracers share packed
+// instructions, four of them a launch's loads of the flow.  Per step,
+// upwind-biased, against mask tests and scalar tracers: 2049^2 with 1, 2, 3, 4
+// tracers 74, 117, 167, 216 us then, 65, 93, 137, 172 now (two: 3.5 TB/s of
+// the 82 B a point); 194 x 92 20, 25, 33, 35 then, 19, 21, 23, 24 now.  Three or
+// four tracers in two launches instead: 157 and 182 us, 39 and 41.
 // PF 1: each iteration also asks L2 for the input rows two beyond those it
 // loads and for the update inputs of the output row after next, so that a
 // state larger than L2 does not make the warp wait on DRAM (trc_prefetch):
 // lanes 2 f and 2 f + 1 ask for the two ends of field f's row segment.
 // Resident blocks per SM asked of the register allocator: 6 with one tracer,
-// 4 with two.
+// 4 with two, 3 with more (none spills).
 template <int NT, int FLUX, int PF>
-__global__ void __launch_bounds__(128, NT == 1 ? 6 : 4) k_trc32(TrcP p, int S, int nstrips) {
-  using V = typename std::conditional<NT == 2, float2, float>::type;
+__global__ void __launch_bounds__(128, NT == 1 ? 6 : NT == 2 ? 4 : 3) k_trc32(TrcP p, int S, int nstrips) {
+  using V = typename Values<NT>::type;
   constexpr int H = 2, TI = 32 - 2 * H;
   const int lane = threadIdx.x & 31;
   // block b: strip b % nstrips, its four warps four consecutive row groups
@@ -190,34 +232,37 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : 4) k_trc32(TrcP p, int S, i
   V pg1 = {}, pg2 = {}, pc0 = {};
   V fyp = {};  // flux through the north faces of the previous output row
 
-  // the lane's prefetches: an input field of row J + 4, or an update input of
-  // output row J
-  const char *pfp = nullptr;
+  // the lane's prefetches, one per two tracers: an input field of row J + 4,
+  // or an update input of output row J
+  constexpr int NP = (NT + 1) / 2;
+  const char *pfp[NP] = {};
   int pfs = 4;
-  bool pfi = false;
+  bool pfi[NP] = {};
   if (PF) {
     const int f = lane >> 1, e = (lane & 1) * 31;
-    const void *b = nullptr;
-    switch (f) {
-      case 0: b = p.mask16; pfs = 2; break;
-      case 1: b = p.He; break;
-      case 2: b = p.nl ? p.eta : nullptr; break;
-      case 3: b = p.u; break;
-      case 4: b = p.v; break;
-      case 5: b = p.t[0].ch; break;
-      case 6: b = p.t[0].cl; break;
-      case 7: b = NT == 2 ? p.t[NT - 1].ch : nullptr; break;
-      case 8: b = NT == 2 ? p.t[NT - 1].cl : nullptr; break;
-      case 9: b = p.t[0].G1; break;
-      case 10: b = p.t[0].G2; break;
-      case 11: b = p.t[0].C0; break;
-      case 12: b = NT == 2 ? p.t[NT - 1].G1 : nullptr; break;
-      case 13: b = NT == 2 ? p.t[NT - 1].G2 : nullptr; break;
-      case 14: b = NT == 2 ? p.t[NT - 1].C0 : nullptr; break;
-      default: break;
+    const int col = ((gx0 + e) % nx + nx) % nx;
+#pragma unroll
+    for (int s = 0; s < NP; s++) {
+      const void *b = nullptr;
+      const int fs = s ? f + 5 : f;  // the flow's fields go with the first two tracers
+      if (s == 0) {
+        if (f == 0) b = p.mask16, pfs = 2;
+        if (f == 1) b = p.He;
+        if (f == 2) b = p.nl ? p.eta : nullptr;
+        if (f == 3) b = p.u;
+        if (f == 4) b = p.v;
+      }
+#pragma unroll
+      for (int q = 2 * s; q < 2 * s + 2 && q < NT; q++) {
+        const int g = fs - 5 - 5 * (q - 2 * s);
+        if (g == 0) b = p.t[q].ch;
+        if (g == 1) b = p.t[q].cl;
+        if (g == 2) b = p.t[q].G1, pfi[s] = true;
+        if (g == 3) b = p.t[q].G2, pfi[s] = true;
+        if (g == 4) b = p.t[q].C0, pfi[s] = true;
+      }
+      if (b) pfp[s] = static_cast<const char *>(b) + (size_t)col * (s ? 4 : pfs);
     }
-    pfi = f >= 9;
-    if (b) pfp = static_cast<const char *>(b) + (size_t)(((gx0 + e) % nx + nx) % nx) * pfs;
   }
 
   auto body = [&](auto fast_tag) {
@@ -252,8 +297,8 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : 4) k_trc32(TrcP p, int S, i
     const V ch = chs[2], chjp = chs[1], chjm = chs[3];
     const V chip = vdown(ch, 1), chim = vup(ch), chrr = FLUX ? vdown(ch, 2) : vb<V>(0.f);
     const V mC = vmul(ch, vb<V>(-ro));  // -C
-    const V fxe = face_flux<FAST, FLUX>(uip, chim, ch, chip, chrr, oUip, oEim, oE, oEip, oEipp);
-    const V fyn = face_flux<FAST, FLUX>(cvp * vjp, chjm, ch, chjp, chs[0], oVjp, oEjm, oE, oEjp, oEjpp);
+    const V fxe = face_flux<FAST, FLUX>(FAST ? uip : (float)oUip * uip, chim, ch, chip, chrr, oEim, oE, oEip, oEipp);
+    const V fyn = face_flux<FAST, FLUX>(FAST ? cvp * vjp : (float)oVjp * cvp * vjp, chjm, ch, chjp, chs[0], oEjm, oE, oEjp, oEjpp);
     const V fys = fyp;
     fyp = fyn;
     const V dxe = vmul(vmul(vfma(chip, vb<V>(rip), mC), vb<V>(huip)), vb<V>(c8));
@@ -315,8 +360,11 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : 4) k_trc32(TrcP p, int S, i
     n1 = n2;
     if (J + 2 < jend) load(J + 2, n2);
     if (PF) {
-      const bool want = pfp && (pfi ? J >= ry0 && J < ylast : J + 4 < jend);
-      if (want) prefetch_l2(pfp + (size_t)(unsigned)(pfi ? off[0] : nx * wr(J + 4, ny)) * pfs);
+#pragma unroll
+      for (int s = 0; s < NP; s++) {
+        const bool want = pfp[s] && (pfi[s] ? J >= ry0 && J < ylast : J + 4 < jend);
+        if (want) prefetch_l2(pfp[s] + (size_t)(unsigned)(pfi[s] ? off[0] : nx * wr(J + 4, ny)) * (s ? 4 : pfs));
+      }
     }
     // row ry0 - 1 only forms its north faces (the south faces of row ry0)
     if (J - 2 >= ry0 - 1) {  // uniform across the warp
@@ -385,7 +433,9 @@ static int trc_resident_nt(const TrcP &p) {
 static void trc_launch(const TrcP &p, int S, cudaStream_t st) {
   switch (p.ntr) {
     case 1: trc_launch_nt<1>(p, S, st); break;
-    default: trc_launch_nt<2>(p, S, st); break;
+    case 2: trc_launch_nt<2>(p, S, st); break;
+    case 3: trc_launch_nt<3>(p, S, st); break;
+    default: trc_launch_nt<4>(p, S, st); break;
   }
 }
 
@@ -393,7 +443,9 @@ static void trc_launch(const TrcP &p, int S, cudaStream_t st) {
 static int trc_resident(const TrcP &p) {
   switch (p.ntr) {
     case 1: return trc_resident_nt<1>(p);
-    default: return trc_resident_nt<2>(p);
+    case 2: return trc_resident_nt<2>(p);
+    case 3: return trc_resident_nt<3>(p);
+    default: return trc_resident_nt<4>(p);
   }
 }
 
