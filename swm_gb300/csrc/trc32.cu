@@ -122,16 +122,17 @@ struct Values<4> { using type = More<float2>; };
 // Advective flux of CH through the face between L and R (R east or north of
 // L, Lm behind L, Rp beyond R) for the velocity vel (times the row's cosine at
 // a north face; 0, or NaN where it is not finite, at a closed face): the
-// third-order upwind-biased value (-1, 5, 2)/6 from the upwind side where all
-// four cells are ocean (FLUX 1), the mask-weighted mean elsewhere.  FAST: all
+// third-order upwind-biased value (-1, 5, 2)/6 from the upwind side (pos: from
+// L; the velocity's sign, not vel's, as grids may reach beyond a pole, where
+// the cosine is negative) where all four cells are ocean (FLUX 1), the
+// mask-weighted mean elsewhere.  FAST: all
 // masks are 1.  The mean's halves are taken before the sum: where a field
 // overflows, which cells hold infinities and NaNs does not depend on the body.
 template <bool FAST, int FLUX, typename V>
-__device__ __forceinline__ V face_flux(float vel, V cLm, V cL, V cR, V cRp, unsigned oLm, unsigned oL, unsigned oR,
-                                       unsigned oRp) {
+__device__ __forceinline__ V face_flux(float vel, bool pos, V cLm, V cL, V cR, V cRp, unsigned oLm, unsigned oL,
+                                       unsigned oR, unsigned oRp) {
   V f;
   if (FLUX == 1) {
-    const bool pos = vel >= 0.f;
     const V kL = vb<V>(pos ? 5.f : 2.f), kR = vb<V>(pos ? 2.f : 5.f);
     const V t = vsub(vfma(kL, cL, vmul(kR, cR)), vsel(pos, cLm, cRp));
     f = vmul(vmul(t, vb<V>(1.f / 6.f)), vb<V>(vel));
@@ -297,8 +298,9 @@ __global__ void __launch_bounds__(128, NT == 1 ? 6 : NT == 2 ? 4 : 3) k_trc32(Tr
     const V ch = chs[2], chjp = chs[1], chjm = chs[3];
     const V chip = vdown(ch, 1), chim = vup(ch), chrr = FLUX ? vdown(ch, 2) : vb<V>(0.f);
     const V mC = vmul(ch, vb<V>(-ro));  // -C
-    const V fxe = face_flux<FAST, FLUX>(FAST ? uip : (float)oUip * uip, chim, ch, chip, chrr, oEim, oE, oEip, oEipp);
-    const V fyn = face_flux<FAST, FLUX>(FAST ? cvp * vjp : (float)oVjp * cvp * vjp, chjm, ch, chjp, chs[0], oEjm, oE, oEjp, oEjpp);
+    const float ue = FAST ? uip : (float)oUip * uip, vn = FAST ? cvp * vjp : (float)oVjp * cvp * vjp;
+    const V fxe = face_flux<FAST, FLUX>(ue, uip >= 0.f, chim, ch, chip, chrr, oEim, oE, oEip, oEipp);
+    const V fyn = face_flux<FAST, FLUX>(vn, vjp >= 0.f, chjm, ch, chjp, chs[0], oEjm, oE, oEjp, oEjpp);
     const V fys = fyp;
     fyp = fyn;
     const V dxe = vmul(vmul(vfma(chip, vb<V>(rip), mC), vb<V>(huip)), vb<V>(c8));
