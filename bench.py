@@ -825,14 +825,15 @@ def reference(args, rank, ws):
 def sor_measurement(args, cells=4096, eps=1e-4):
     """The reference's own solver (main_ElSolv_SOR: masked spherical
     Laplacian, fixed Chebyshev relaxation schedule, absolute stop on the
-    correction norm, eps = 1e-4 as calc_lib.h) on the 4096^2 basin (chi, B,
-    the five coefficients and the reciprocal diagonal, 1.3 GB, exceed L2).  The right-hand side is a
+    correction norm, eps = 1e-4 as calc_lib.h) on the 4096^2 basin (two
+    buffers of chi, B and the mask bits, 0.42 GB, exceed L2).  The right-hand side is a
     smooth random field of the size of a flow divergence (1e-9 /s), as
     computeVelocityPotential passes one.  A call after the first (first_guess
     false, as every call but the first from the diagnostics) is capped by the
     reference at max_count = 10 max(Nx, Ny) iterations; from chi = 0 it may
-    end there unconverged, which is reported.  Roofline: 10 words per point and iteration (chi read
-    and written, B, the five coefficients, the reciprocal diagonal)."""
+    end there unconverged, which is reported.  Roofline: 33 B per point and iteration (chi of both
+    colours read, chi written, B, a byte of mask bits; the coefficients depend
+    on the row and the mask case)."""
     import torch
     from swm_gb300.host import synthetic
     from swm_gb300.host.driver import Driver
@@ -863,17 +864,17 @@ def sor_measurement(args, cells=4096, eps=1e-4):
     it = abs(iters)
     pts = nx * ny
     peak, kind = peaks()
-    ach = 10 * 8 * pts * it / dev / 1e9
+    ach = 33 * pts * it / dev / 1e9
     g.close()
     return {'workload': 'elsolv_sor_%dx%d' % (cells, cells), 'points': pts, 'eps': eps,
             'iterations': it, 'converged': iters > 0, 'anorm': anorm, 'max_count': 10 * max(nx, ny),
             'time_s': wall, 'device_s': dev, 'ms_per_iteration': dev / max(it, 1) * 1e3,
             'gpu_launches': launches,
             'roofline': {'bound': 'hbm', 'achieved': ach, 'peak': peak, 'unit': 'GB/s', 'frac': ach / peak,
-                         'peak_kind': kind, 'bytes_per_point_iteration': 80,
+                         'peak_kind': kind, 'bytes_per_point_iteration': 33,
                          'note': 'one iteration = a red and a black half-sweep over all points; the half-sweep '
                                  "is bound by GB300's FP64 pipe: the reference's update is FP64 arithmetic, "
-                                 'its division formed from the reciprocal diagonal by Markstein corrections'}}
+                                 'its division formed in two operations from a two-word reciprocal diagonal'}}
 
 
 def main():
