@@ -2,9 +2,9 @@
 // without the gap of a launch.  The FP32 step kernel waits for its predecessor
 // at its start and then lets its successor launch (whose blocks take the places
 // that finished blocks leave): 65^2 step 5.1 -> 4.8 us, 1025^2 30.4 us before and
-// 30.0 after.  The FP64 step kernels do not: with several models stepped at
-// once, blocks that wait kept others from running (257 x 129 points 9.9 -> 13.6
-// us a step), and a single model gained 1 us of 17.
+// 30.0 after.  The plain path's kernels do not: with three models
+// stepped at once, blocks that wait kept others from running (257 x 129 points
+// 8.4 -> 10.0 us a step; 61^2, which leaves places free, gained 8 %).
 #pragma once
 #include <cuda_runtime.h>
 
