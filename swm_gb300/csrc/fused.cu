@@ -62,6 +62,7 @@ struct FusedState {
   void *Fc[3] = {};
   double *ms_zeta = nullptr, *ms_ex = nullptr;
   Scratch64 s64;  // FP64 path
+  FixedDiv impl_d[3] = {};
 };
 
 namespace swm {
@@ -151,6 +152,8 @@ int fused_prepare(swm_gpu_ctx *c) {
   for (int q = 0; q < 3; q++) f->impl_uniform = f->impl_uniform && uniform(g.impl[q], &f->impl_s[q]);
   if (!f->impl_uniform)
     for (int q = 0; q < 3; q++) FTRY(upload_t(c, f32, g.impl[q].data(), n, &f->impl[q]));
+  else if (!f32)
+    FTRY(fused64_divisors(c, f->impl_s, 3, f->impl_d));
   f->gsq_uniform = uniform(g.gsq[0], &f->gsq_s[0]) && uniform(g.gsq[1], &f->gsq_s[1]);
   if (!f->gsq_uniform)
     for (int q = 0; q < 2; q++) FTRY(upload_t(c, f32, g.gsq[q].data(), n, &f->gsq[q]));
@@ -362,7 +365,7 @@ static void make_p64(swm_gpu_ctx *c, int64_t itt, P64 &p) {
   p.lbc = cf.lbc;
   p.q1 = 1. / (cf.A * c->hg.dTheta);
   p.ts_rho = cf.tau_scale / cf.RHO0;
-  for (int q = 0; q < 3; q++) p.dp_s[q] = (f->impl_s[q] - 1.) / f->impl_s[q];
+  for (int q = 0; q < 3; q++) p.impl_d[q] = f->impl_d[q];
   for (int q = 0; q < 2; q++) p.gsq_s[q] = f->gsq_s[q];
   p.mc = f->mc;
   p.He = (const double *)f->He;

@@ -9,8 +9,8 @@
 // whose tiles of 32 x 8 recompute two halo cells took 615 us there.  Masks are
 // selects, metric factors and mask cases per-row tables, a thickness that
 // divides is inverted once (three fused operations on the hardware's seed),
-// and the implicit damping is x - x dp with dp = 1 - 1/impl, so that its
-// rounding does not depend on 1/impl's.  About 86 operations per point
+// and a uniform implicit damping factor divides as a fixed divisor
+// (divide.cuh).  About 86 operations per point
 // (Laplacian), 104 (biharmonic).
 //
 // 1025 x 1025, biharmonic: 615 -> 230 us per step.
@@ -277,10 +277,12 @@ __global__ void __launch_bounds__(256) k_f64_step(P64 p) {
   p.Ge3[k] = ge;
   p.Gu3[k] = gu;
   p.Gv3[k] = gv;
+  // a uniform factor is a fixed divisor: two operations, the division's quotient (x / 1 = x)
   auto next = [&](double x, const double *G1, const double *G2, double g, int f) {
     x += p.ab0 * G1[k] + p.ab1 * G2[k] + p.ab2 * g;
     if (!p.impl_uniform) return x / p.impl[f][k];
-    return p.dp_s[f] != 0. ? x - x * p.dp_s[f] : x;
+    const FixedDiv &d = p.impl_d[f];
+    return __double_as_longlong(d.b) == 0x3ff0000000000000ll ? x : div_fixed(x, d);
   };
   double e1 = next(e, p.Ge1, p.Ge2, ge, 2);
   if (p.nl) {
@@ -295,6 +297,24 @@ __global__ void __launch_bounds__(256) k_f64_step(P64 p) {
 #undef POINT64
 
 }  // namespace
+
+__global__ void k_f64_divisor(double b, FixedDiv *out) { *out = fixed_div(b); }
+
+int fused64_divisors(swm_gpu_ctx *c, const double *b, int count, FixedDiv *out) {
+  FixedDiv *d = nullptr;
+  if (cudaMalloc((void **)&d, count * sizeof(FixedDiv)) != cudaSuccess) {
+    set_error("fused64: cudaMalloc failed");
+    return SWM_GPU_ENOMEM;
+  }
+  for (int q = 0; q < count; q++) k_f64_divisor<<<1, 1, 0, c->stream>>>(b[q], d + q);
+  c->launches += count;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, count * sizeof(FixedDiv), cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  cudaFree(d);
+  SWM_CK(e);
+  return SWM_GPU_OK;
+}
 
 int fused64_launch(swm_gpu_ctx *c, const P64 &p) {
   const dim3 b(32, 8), g((c->nx + 31) / 32, (c->ny + 7) / 8);

@@ -3,6 +3,7 @@
 #pragma once
 #include <vector>
 #include "ctx.h"
+#include "divide.cuh"
 
 namespace swm {
 
@@ -36,7 +37,8 @@ struct P64 {
   int nx, ny, nl, has_mode, mix, qbf, barotropic, has_F, impl_uniform, gsq_uniform, wind_x, wind_y, wind_rows;
   double G, lbc, q1, ts_rho, minD;
   double ab0, ab1, ab2;  // Adams-Bashforth weights times dt
-  double dp_s[3], gsq_s[2];
+  FixedDiv impl_d[3];  // uniform damping factors
+  double gsq_s[2];
   const uint8_t *mc;  // mask code: bit 0 H, 1 u, 2 v, 3 eta
   const double *He, *rows, *Hu, *Hv;
   const double *impl[3], *gsq[2];
@@ -48,6 +50,8 @@ struct P64 {
   double *Gu3, *Gv3, *Ge3;
   Scratch64 s;
 };
+// b as fixed divisors
+int fused64_divisors(swm_gpu_ctx *c, const double *b, int count, FixedDiv *out);
 int fused64_launch(swm_gpu_ctx *c, const P64 &p);
 
 }  // namespace swm

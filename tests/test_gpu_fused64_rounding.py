@@ -1,0 +1,57 @@
+"""fused_fp64 divides: by a uniform damping factor, by the thickness (wind
+stress, potential vorticity).  Each quotient is compared at points where
+everything else in it is exact, or where the rest is far smaller."""
+import numpy as np
+import pytest
+
+from harness import run_case
+from swm_gb300.host import synthetic
+from swm_gb300.model import GpuModel
+
+pytestmark = pytest.mark.gpu
+
+
+def one_step(case, path='fused_fp64'):
+    g = GpuModel(path)
+    run_case(case, g, nsteps=1, with_diag=False)
+    return g
+
+
+def uniform_damping(gamma):
+    return [dict(term=t, type=0, value=gamma, sl_length=1.0, sl_cutoff=15.0, loc=0, file_data=None) for t in (0, 1)]
+
+
+@pytest.mark.parametrize('strength', [1e-3, 1.0, 1e6, 1e12])
+def test_uniform_damping_keeps_its_digits(strength):
+    """u / (1 + dt gamma), dt gamma = strength, against plain_fp64.  A step of
+    1e-3 s changes u (0.5 to 1.5 m/s) by less than 1e-6, so that the tendency's
+    roundings are below 1e-6 x 64 x 2^-53 of it: the two sums are at most one
+    ulp apart and each quotient half an ulp off, 2 ulps or 4 x 2^-53 together."""
+    dt = 1e-3
+    case = synthetic.double_gyre((45, 37), biharmonic=False, dt=dt, nsteps=1)
+    case['damping'] = uniform_damping(strength / dt)
+    rng = np.random.default_rng(4)
+    H = case['H']
+    case['ic'] = {f: rng.choice([-1.0, 1.0], H.shape) * (0.5 + rng.random(H.shape)) for f in ('u', 'v')}
+    a, b = one_step(case), one_step(case, 'plain_fp64')
+    for f in ('u', 'v'):
+        x, y, m = a.field(f), b.field(f), a.ocean(f).astype(bool)
+        assert (y[m] != 0).all()
+        assert (np.abs(x - y)[m] <= 4 * 2.0 ** -53 * np.abs(y)[m]).all()
+    a.close()
+    b.close()
+
+
+def test_infinite_velocity_under_uniform_damping():
+    """An infinite velocity stays infinite under a finite damping factor: u holds
+    its infinity where plain_fp64's does, and no NaN."""
+    case = synthetic.linear_rg(40, 24, nsteps=1)
+    case['config'].update(lateral_mixing=0)
+    case['ic'] = {f: np.zeros_like(case['H']) for f in ('u', 'v', 'eta')}
+    case['ic']['u'][6, 20] = np.inf
+    a, b = one_step(case), one_step(case, 'plain_fp64')
+    x, y = a.field('u'), b.field('u')
+    assert np.isinf(y[6, 20]) and not np.isnan(y).any()
+    assert np.array_equal(np.isinf(x), np.isinf(y)) and not np.isnan(x).any()
+    a.close()
+    b.close()
