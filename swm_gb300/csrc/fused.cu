@@ -135,7 +135,7 @@ int fused_prepare(swm_gpu_ctx *c) {
     FTRY(upload_t(c, false, rows.data(), rows.size(), &f->rows));
     const int mix = cf.lateral_mixing ? (cf.mixing_kind == SWM_MIX_BIHARMONIC ? 2 : 1) : 0;
     Scratch64 &s = f->s64;
-    double **bufs[] = {&s.mu, &s.mv, &s.pot, &s.B, &s.rdu, &s.rdv, &s.pl, &s.pt, &s.dh, &s.lu, &s.lv};
+    double **bufs[] = {&s.mu, &s.mv, &s.pot, &s.B, &s.du, &s.dv, &s.pl, &s.pt, &s.dh, &s.lu, &s.lv};
     const int nb = mix == 2 ? 11 : (mix == 1 ? 8 : 6);
     for (int q = 0; q < nb; q++) FTRY(dmalloc((void **)bufs[q], n * 8));
   }
@@ -787,7 +787,7 @@ void fused_free(swm_gpu_ctx *c) {
   for (int q = 0; q < 3; q++) { F(f->dp[q]); F(f->Fc[q]); }
   F(f->ms_zeta); F(f->ms_ex);
   Scratch64 &s = f->s64;
-  F(s.mu); F(s.mv); F(s.pot); F(s.B); F(s.rdu); F(s.rdv); F(s.pl); F(s.pt); F(s.dh); F(s.lu); F(s.lv);
+  F(s.mu); F(s.mv); F(s.pot); F(s.B); F(s.du); F(s.dv); F(s.pl); F(s.pt); F(s.dh); F(s.lu); F(s.lv);
   delete f;
   c->fused = nullptr;
 }

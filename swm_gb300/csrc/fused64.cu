@@ -7,10 +7,9 @@
 // passes therefore form every quantity once per point and hand it on through
 // memory, instead of rebuilding it in the halo of a tile: a one-kernel step
 // whose tiles of 32 x 8 recompute two halo cells took 615 us there.  Masks are
-// selects, metric factors and mask cases per-row tables, a thickness that
-// divides is inverted once (three fused operations on the hardware's seed),
-// and a uniform implicit damping factor divides as a fixed divisor
-// (divide.cuh).  About 86 operations per point
+// selects, metric factors and mask cases per-row tables, stress and wind are
+// added before they are divided by the thickness, and a uniform implicit
+// damping factor divides as a fixed divisor (divide.cuh).  About 86 operations per point
 // (Laplacian), 104 (biharmonic).
 //
 // 1025 x 1025, biharmonic: 615 -> 230 us per step.
@@ -93,18 +92,6 @@ __device__ __forceinline__ double inv_count(int n) { return n >= 4 ? .25 : (n ==
 // mask case of a stress coefficient with own bit a and other bit b
 __device__ __forceinline__ int mcase(int a, int b) { return a ? 1 + b : 0; }
 
-// 1 / x: from the hardware's seed y (its error e = 1 - x y is below 2^-18) by
-// y (1 + e + e^2), whose error is e^3 besides rounding; magnitudes outside
-// [2^-500, 2^500] (0, infinities and NaN among them) divide
-__device__ __forceinline__ double recip(double x) {
-  const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (ex - 523u > 1000u) return 1. / x;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.);
-  return fma(y, fma(e, e, e), y);
-}
-
 // a < b; the doubles' order as integers decides, and FP64 only confirms
 __device__ __forceinline__ bool less(double a, double b) {
   long long x = __double_as_longlong(a), y = __double_as_longlong(b);
@@ -152,8 +139,8 @@ __device__ __forceinline__ double div_v(const double *r, const At &q, unsigned m
   const double *r = p.rows + (size_t)q.j * R_NR;        \
   const unsigned m = p.mc[k];
 
-// mass fluxes, potential vorticity, Bernoulli potential, reciprocal
-// thicknesses and the (first) stress pass
+// mass fluxes, potential vorticity, Bernoulli potential, thicknesses that the
+// step divides by and the (first) stress pass
 template <int MIX>
 __global__ void __launch_bounds__(256) k_f64_diag(P64 p) {
   POINT64
@@ -172,8 +159,8 @@ __global__ void __launch_bounds__(256) k_f64_diag(P64 p) {
   const double Dh = (dwd + (ds + dsw)) * inv_count(a + b + c + x);
   p.s.mu[k] = mU(m) ? Du * u : 0.;
   p.s.mv[k] = mV(m) ? Dv * v : 0.;
-  if (MIX || p.wind_x) p.s.rdu[k] = mU(m) ? recip(Du) : 0.;
-  if (MIX || p.wind_y) p.s.rdv[k] = mV(m) ? recip(Dv) : 0.;
+  if (MIX || p.wind_x) p.s.du[k] = Du;
+  if (MIX || p.wind_y) p.s.dv[k] = Dv;
   double pot = 0., B = 0.;
   if (p.has_mode) {
     double z = r[R_FH];
@@ -187,7 +174,7 @@ __global__ void __launch_bounds__(256) k_f64_diag(P64 p) {
       if (mV(m) | mV(mw)) z += dv;
       if (mU(m) | mU(ms)) z += du;
     }
-    pot = z * recip(at_least_eps(Dh));
+    pot = z / at_least_eps(Dh);
     if (mE(m)) {
       B = p.G * e;
       if (p.nl) {
@@ -253,7 +240,7 @@ __global__ void __launch_bounds__(256) k_f64_step(P64 p) {
     if (MIX || p.wind_x) {
       double t = MIX ? div_u(r, q, m, mn, p.s.pl, p.s.pt) : 0.;
       if (p.wind_x) t += p.ts_rho * (p.wind_rows ? p.wx[q.j] : p.wx[k]);
-      g += t * p.s.rdu[k];
+      g += t / p.s.du[k];
     }
     if (p.has_F) g += p.Fx[k];
     gu = g;
@@ -269,7 +256,7 @@ __global__ void __launch_bounds__(256) k_f64_step(P64 p) {
     if (MIX || p.wind_y) {
       double t = MIX ? div_v(r, q, m, ms, p.s.pl, p.s.pt) : 0.;
       if (p.wind_y) t += p.ts_rho * (p.wind_rows ? p.wy[q.j] : p.wy[k]);
-      g += t * p.s.rdv[k];
+      g += t / p.s.dv[k];
     }
     if (p.has_F) g += p.Fy[k];
     gv = g;

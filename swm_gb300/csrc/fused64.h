@@ -28,7 +28,7 @@ std::vector<double> fused64_rows(const swm_gpu_ctx *c);
 // what the passes of a step hand on, one value per point
 struct Scratch64 {
   double *mu = nullptr, *mv = nullptr, *pot = nullptr, *B = nullptr;  // mass fluxes, PV / 8, Bernoulli potential
-  double *rdu = nullptr, *rdv = nullptr;                   // 1 / thickness at u and v points
+  double *du = nullptr, *dv = nullptr;                     // thickness at u and v points
   double *pl = nullptr, *pt = nullptr;                     // stress
   double *dh = nullptr, *lu = nullptr, *lv = nullptr;      // biharmonic: thickness at H points, first-pass divergence
 };

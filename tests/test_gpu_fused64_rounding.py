@@ -55,3 +55,67 @@ def test_infinite_velocity_under_uniform_damping():
     assert np.array_equal(np.isinf(x), np.isinf(y)) and not np.isnan(x).any()
     a.close()
     b.close()
+
+
+def wet_surroundings(H, r=3):
+    """Points whose neighbours up to r cells away are all ocean."""
+    m = H > 0
+    for axis in (0, 1):
+        m = np.logical_and.reduce([np.roll(m, s, axis) for s in range(-r, r + 1)])
+    return m
+
+
+def integer_depths(shape):
+    """A box of depths H that are whole multiples of 32 m: their means at the
+    eta points (D) and the means of two and of four of those are exact."""
+    H = 32.0 * np.random.default_rng(6).integers(5, 50, shape)
+    H[:, 0] = H[:, -1] = H[0] = H[-1] = 0.0
+    return H
+
+
+def west(a):
+    return np.roll(a, 1, 1)
+
+
+def south(a):
+    return np.roll(a, 1, 0)
+
+
+def north(a):
+    return np.roll(a, -1, 0)
+
+
+def test_wind_over_thickness_is_the_quotient():
+    """From rest, the tendency of u is tau / rho0 over the thickness: the
+    quotient of the two, correctly rounded (rho0 is a power of two)."""
+    case = synthetic.double_gyre((65, 49), biharmonic=False, nsteps=1)
+    case['config'].update(lateral_mixing=0)
+    case['H'] = integer_depths(case['H'].shape)
+    case['damping'] = []
+    g = one_step(case)
+    m = wet_surroundings(case['H'])
+    D = g.field('D')
+    want = case['streams'][0]['rec1'][0] / case['config']['RHO0'] / np.where(m, 0.5 * (D + west(D)), 1.0)
+    assert m.sum() > 1000 and np.array_equal(g.field('G_u')[m], want[m])
+    g.close()
+
+
+def test_potential_vorticity_is_the_quotient():
+    """Linear, u = eta = 0, v a whole number: the tendency of u is
+    (f/D + f/D) / 2 times the mean mass flux.  With f over 8 the quotients are
+    one rounding each, their sum one and its product with the (whole) sum of
+    four mass fluxes one."""
+    case = synthetic.linear_rg(64, 48, nsteps=1)
+    H = case['H'] = integer_depths(case['H'].shape)
+    case['config'].update(lateral_mixing=0, H_overwrite=0.0)
+    case['damping'] = []
+    case['ic'] = {'v': np.random.default_rng(7).integers(-3, 4, H.shape).astype(float)}
+    g = one_step(case)
+    D, v = g.field('D'), case['ic']['v'] * g.ocean('v')
+    Dh = 0.25 * ((D + west(D)) + (south(D) + south(west(D))))
+    pot = (g.lat('f_H') / 8)[:, None] / np.where(Dh > 0, Dh, 1.0)
+    mv = 0.5 * (D + south(D)) * v
+    want = (north(pot) + pot) * ((north(mv) + west(mv)) + (north(west(mv)) + mv))
+    m = wet_surroundings(H)
+    assert m.sum() > 1000 and np.array_equal(g.field('G_u')[m], want[m])
+    g.close()
