@@ -7,12 +7,13 @@
 // passes therefore form every quantity once per point and hand it on through
 // memory, instead of rebuilding it in the halo of a tile: a one-kernel step
 // whose tiles of 32 x 8 recompute two halo cells took 615 us there.  Masks are
-// selects, metric factors and mask cases per-row tables, stress and wind are
+// selects, metric factors and mask cases per-row tables (of a difference, not
+// of its two terms, whose roundings would not cancel), stress and wind are
 // added before they are divided by the thickness, and a uniform implicit
 // damping factor divides as a fixed divisor (divide.cuh).  About 86 operations per point
 // (Laplacian), 104 (biharmonic).
 //
-// 1025 x 1025, biharmonic: 615 -> 230 us per step.
+// 1025 x 1025, biharmonic: 615 -> 252 us per step.
 //
 // Formulas: swm_nonlinear_timestep_module.f90:182-449 (diagnostics and
 // tendencies), swm_lateralmixing_module.f90:66-240 (stress), time_integration_
@@ -34,11 +35,13 @@ std::vector<double> fused64_rows(const swm_gpu_ctx *c) {
     const double cE = g.cosl[GE][j], cU = g.cosl[GU][j], cV = g.cosl[GV][j], cH = g.cosl[GH][j];
     r[R_FH] = g.f[GH][j] / 8.;
     r[R_ZV] = 1. / (A * cH * dL) / 8.;
-    r[R_ZU] = cU / (A * dT * cH) / 8.;
-    r[R_ZUM] = g.cosl[GU][jm] / (A * dT * cH) / 8.;
+    r[R_ZU] = 1. / (A * dT * cH) / 8.;
+    r[R_CU] = cU;
+    r[R_CUM] = g.cosl[GU][jm];
     r[R_EX] = 1. / (A * cE * dL);
-    r[R_EY0] = cV / (A * cE * dT);
-    r[R_EY1] = g.cosl[GV][jp] / (A * cE * dT);
+    r[R_EY] = 1. / (A * cE * dT);
+    r[R_CV] = cV;
+    r[R_CVP] = g.cosl[GV][jp];
     r[R_RU] = 1. / (A * cU * dL);
     for (int pass = 0; pass < 2; pass++) {
       // biharmonic: unit coefficient, then -bih; else the only pass
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(256) k_f64_diag(P64 p) {
     double z = r[R_FH];
     if (p.nl) {
       const double us = p.u0[q.s], vw = p.v0[q.w];
-      double dv = r[R_ZV] * (v - vw), du = r[R_ZUM] * us - r[R_ZU] * u;
+      double dv = r[R_ZV] * (v - vw), du = r[R_ZU] * (r[R_CUM] * us - r[R_CU] * u);
       if (!mH(m)) {
         dv *= p.lbc;
         du *= p.lbc;
@@ -226,7 +229,7 @@ __global__ void __launch_bounds__(256) k_f64_step(P64 p) {
   const double e = p.e0[k], u = p.u0[k], v = p.v0[k];
   double ge = 0., gu = 0., gv = 0.;
   if (mE(m)) {
-    ge = r[R_EX] * (mu[k] - mu[q.e]) + r[R_EY0] * mv[k] - r[R_EY1] * mv[q.n];
+    ge = r[R_EX] * (mu[k] - mu[q.e]) + r[R_EY] * (r[R_CV] * mv[k] - r[R_CVP] * mv[q.n]);
     if (p.has_F) ge += p.Fe[k];
   }
   if (mU(m)) {

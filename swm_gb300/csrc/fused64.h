@@ -13,8 +13,10 @@ namespace swm {
 enum {
   R_FH,                           // f / 8 (the potential vorticity is kept divided by 8, the weight
                                   // 1/2 * 1/4 of its product with the mass flux)
-  R_ZV, R_ZU, R_ZUM,              // vorticity: 1/(A cosH dL), cosU_j/(A dT cosH_j), cosU_{j-1}/(A dT cosH_j), over 8
-  R_EX, R_EY0, R_EY1,             // continuity: 1/(A cosE dL), cosV_j/(A cosE dT), cosV_{j+1}/(A cosE dT)
+  R_ZV, R_ZU,                     // vorticity: 1/(A cosH dL), 1/(A dT cosH), over 8
+  R_CU, R_CUM,                    // cosU_j, cosU_{j-1}
+  R_EX, R_EY,                     // continuity: 1/(A cosE dL), 1/(A cosE dT)
+  R_CV, R_CVP,                    // cosV_j, cosV_{j+1}
   R_RU,                           // 1/(A cosU dL)
   R_P0, R_P1, R_P2 = R_P1 + 3,    // stress at eta points
   R_H0 = R_P2 + 3, R_H1, R_H2 = R_H1 + 3,  // stress at H points

@@ -119,3 +119,23 @@ def test_potential_vorticity_is_the_quotient():
     m = wet_surroundings(H)
     assert m.sum() > 1000 and np.array_equal(g.field('G_u')[m], want[m])
     g.close()
+
+
+@pytest.mark.parametrize('flow,tendency', [('u', 'G_v'), ('v', 'G_eta')])
+def test_uniform_flow_differences_cancel(flow, tendency):
+    """A uniform flow of 1 m/s over 512 m without rotation: what is left of
+    divergence and vorticity is the change of cos(lat) from row to row, whose
+    products and differences are exact.  At most four roundings follow on
+    fused_fp64 and three on plain_fp64 (powers of two aside), each 2^-53."""
+    case = synthetic.double_gyre((45, 37), biharmonic=False, nsteps=1)
+    case['config'].update(lateral_mixing=0, OMEGA=0.0)
+    case['H'] = np.where(np.pad(np.ones((36, 44)), 1) > 0, 512.0, 0.0)
+    case['damping'], case['streams'] = [], []
+    case['ic'] = {flow: np.ones_like(case['H'])}
+    a, b = one_step(case), one_step(case, 'plain_fp64')
+    m = wet_surroundings(case['H'])
+    x, y = a.field(tendency)[m], b.field(tendency)[m]
+    assert m.sum() > 500 and (y != 0).mean() > 0.9   # (0 where two rows are as far from the equator)
+    assert (np.abs(x - y) <= 8 * 2.0 ** -53 * np.abs(y)).all()
+    a.close()
+    b.close()
