@@ -198,7 +198,8 @@ int swm_gpu_run_monitor(swm_gpu_ctx *ctx, int64_t itt0, int64_t nsteps, int stre
 
 /* ---- host access (the registry pointers the diagnostics read) ---- */
 int swm_gpu_get_field(swm_gpu_ctx *ctx, int field, double *host_out);
-/* swm_gpu_set_field: the state (u, v, eta) at any time; static fields
+/* swm_gpu_set_field: the state (u, v, eta) and its newest increments (G_u,
+   G_v, G_eta) at any time; static fields
    (depths, damping and drag factors, constant forcing, basic state) at any
    time on the plain path, and before the first step on the fused paths
    (SWM_GPU_EINVAL afterwards: those paths keep their own copies). */

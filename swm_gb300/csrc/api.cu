@@ -848,7 +848,7 @@ int swm_gpu_set_field(swm_gpu_ctx *c, int f, const double *in) {
   TRY(h2d(c, p, in, c->n));
   SWM_CK(cudaStreamSynchronize(c->stream));
   c->stress_ready = false;  // the plain path forms the stress of the next step again
-  if (c->cfg.path != SWM_PATH_PLAIN_FP64 && c->stage >= 5 && f <= SWM_F_ETA) TRY(fused_load_field(c, f));
+  if (c->cfg.path != SWM_PATH_PLAIN_FP64 && c->stage >= 5) TRY(fused_load_field(c, f));
   // the plain path forms its reciprocals of the damping factors again, in the
   // linear modes those of the thickness and the potential vorticity too
   const bool linear = c->cfg.mode == SWM_MODE_LIN_REST || c->cfg.mode == SWM_MODE_LIN_MEAN;

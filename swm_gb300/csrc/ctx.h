@@ -225,7 +225,7 @@ int fused_prepare(swm_gpu_ctx *c);
 int fused_step(swm_gpu_ctx *c, int64_t itt);
 int fused_sync_state(swm_gpu_ctx *c);    // FP32 pair state -> FP64 buffers
 int fused_load_state(swm_gpu_ctx *c);    // FP64 buffers -> FP32 pair state
-int fused_load_field(swm_gpu_ctx *c, int field);  // the same for one of u, v, eta
+int fused_load_field(swm_gpu_ctx *c, int field);  // the same for one field the host set
 // fused_sync_state for what one field's read needs, or that field straight into `to`
 int fused_sync_field(swm_gpu_ctx *c, int field, double *to = nullptr, bool *done = nullptr);
 int fused_refresh_wind(swm_gpu_ctx *c, int id);  // stream id's record changed

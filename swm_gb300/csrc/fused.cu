@@ -274,16 +274,22 @@ int fused_load_state(swm_gpu_ctx *c) {
   return SWM_GPU_OK;
 }
 
-// one field (SWM_F_U, _V, _ETA) of the FP64 buffers -> the pair state's
-// current level, for a state the host set; the increments stay
+// one field of the FP64 buffers that the host set -> the pair state: u, v, eta
+// its current level, G_u, G_v, G_eta its newest increment; the others stay
 int fused_load_field(swm_gpu_ctx *c, int field) {
   FusedState *f = c->fused;
   if (!f || !f->ready || !f->comp) return SWM_GPU_OK;
-  const int a = f->n0;
+  const int a = f->n0, g = (f->g0 + 1) % 3, cg = (c->g0 + 1) % 3;
   const unsigned nb = (unsigned)((c->n + 255) / 256);
-  if (field == SWM_F_U) k_split<<<nb, 256, 0, c->stream>>>(c->u[c->n0], f->uh[a], f->ul[a], c->n);
-  else if (field == SWM_F_V) k_split<<<nb, 256, 0, c->stream>>>(c->v[c->n0], f->vh[a], f->vl[a], c->n);
-  else k_split<<<nb, 256, 0, c->stream>>>(c->eta[c->n0], f->eh[a], f->el[a], c->n);
+  switch (field) {
+    case SWM_F_U: k_split<<<nb, 256, 0, c->stream>>>(c->u[c->n0], f->uh[a], f->ul[a], c->n); break;
+    case SWM_F_V: k_split<<<nb, 256, 0, c->stream>>>(c->v[c->n0], f->vh[a], f->vl[a], c->n); break;
+    case SWM_F_ETA: k_split<<<nb, 256, 0, c->stream>>>(c->eta[c->n0], f->eh[a], f->el[a], c->n); break;
+    case SWM_F_GU: k_to_f32<<<nb, 256, 0, c->stream>>>(c->Gu[cg], f->Gu[g], c->n); break;
+    case SWM_F_GV: k_to_f32<<<nb, 256, 0, c->stream>>>(c->Gv[cg], f->Gv[g], c->n); break;
+    case SWM_F_GETA: k_to_f32<<<nb, 256, 0, c->stream>>>(c->Ge[cg], f->Ge[g], c->n); break;
+    default: return SWM_GPU_OK;
+  }
   c->launches++;
   SWM_CK(cudaGetLastError());
   return SWM_GPU_OK;
