@@ -774,7 +774,9 @@ int swm_gpu_get_field_async(swm_gpu_ctx *c, int f, double *out, int64_t *ticket)
   // field beside other kernels, where a kernel's writes hold SMs for as long
   // (8.4 MB fields of a 1025^2 basin, 96 steps and three fields: 2.62 ms with
   // copies, 2.67 without)
-  double *view = c->cfg.path == SWM_PATH_FUSED_FP32C && c->n * 8 <= ((size_t)1 << 20) ? mapped_view(out) : nullptr;
+  const bool small = c->cfg.path == SWM_PATH_FUSED_FP32C && c->n * 8 <= ((size_t)1 << 20);
+  // (a kernel stores whole doubles: an array that is not aligned to them is copied)
+  double *view = small && ((uintptr_t)out & 7) == 0 ? mapped_view(out) : nullptr;
   if (view && mapped_view(out + c->n - 1) != view + c->n - 1) view = nullptr;  // pinned to its end
   bool done = false;
   if (view && c->stage >= 5) TRY(fused_sync_field(c, f, view, &done));
