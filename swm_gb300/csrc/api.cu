@@ -851,14 +851,17 @@ int swm_gpu_set_field(swm_gpu_ctx *c, int f, const double *in) {
   SWM_CK(cudaStreamSynchronize(c->stream));
   c->stress_ready = false;  // the plain path forms the stress of the next step again
   if (c->cfg.path != SWM_PATH_PLAIN_FP64 && c->stage >= 5) TRY(fused_load_field(c, f));
-  // the plain path forms its reciprocals of the damping factors again, in the
-  // linear modes those of the thickness and the potential vorticity too
+  // what the plain path keeps of the fields that do not change in a run: the
+  // reciprocals of the damping factors, in the linear modes also those of the
+  // thickness at the u and v points (the grid's H_u, H_v) and the potential
+  // vorticity (of H on the H points and the basic state's vorticity)
   const bool linear = c->cfg.mode == SWM_MODE_LIN_REST || c->cfg.mode == SWM_MODE_LIN_MEAN;
-  if (f == SWM_F_IMPL_U || f == SWM_F_IMPL_V || f == SWM_F_IMPL_ETA || (linear && f > SWM_F_ETA)) {
-    c->pdiv_ready = false;
-    c->pot_ready = false;
-    invalidate_graph(c);
-  }
+  const bool impl = f == SWM_F_IMPL_U || f == SWM_F_IMPL_V || f == SWM_F_IMPL_ETA;
+  const bool depth = linear && (f == SWM_F_DU || f == SWM_F_DV || f == SWM_F_HU || f == SWM_F_HV);
+  const bool pot = linear && (f == SWM_F_POT || f == SWM_F_DH || f == SWM_F_H || f == SWM_F_ZETA_BS);
+  if (impl || depth) c->pdiv_ready = false;
+  if (pot) c->pot_ready = false;
+  if (impl || depth || pot) invalidate_graph(c);
   return SWM_GPU_OK;
 }
 
