@@ -47,6 +47,7 @@
 // 513 x 513, the same from 1025 x 769 on.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <string>
 #include <vector>
 #include "ctx.h"
@@ -476,6 +477,20 @@ using namespace swm;
 
 extern "C" {
 
+// at most `blocks` blocks with equal spans of cells, of no more threads than
+// cells of a colour (and the warp that adds the norms)
+static void sor_blocks(SorState *s, size_t ns, int blocks) {
+  s->span = (unsigned)std::max<size_t>(32, (ns + blocks - 1) / blocks);
+  s->blocks = (int)((ns + s->span - 1) / s->span);
+  s->threads = (int)std::min<size_t>(SOR_CELL_THREADS, ((size_t)s->span + 31) / 32 * 32) + 32;
+}
+
+// a whole number from the environment, 0 when unset or not positive
+static int sor_env(const char *name) {
+  const char *e = getenv(name);
+  return e && atoi(e) > 0 ? atoi(e) : 0;
+}
+
 int elsolv_sor_gpu_init(swm_gpu_ctx *c) {
   SWM_ON_DEVICE(c ? c->device : -1);
   SWM_REQUIRE(c && c->stage >= 1, "elsolv_sor_gpu_init: call after swm_gpu_domain");
@@ -489,11 +504,9 @@ int elsolv_sor_gpu_init(swm_gpu_ctx *c) {
   s->W = W;
   int sms = 0;
   SWM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device < 0 ? 0 : c->device));
-  // one block per SM, of no more threads than cells of a colour (and the warp
-  // that adds the norms)
-  s->span = (unsigned)std::max<size_t>(32, (ns + sms - 1) / sms);
-  s->blocks = (int)((ns + s->span - 1) / s->span);
-  s->threads = (int)std::min<size_t>(SOR_CELL_THREADS, ((size_t)s->span + 31) / 32 * 32) + 32;
+  // one block per SM, or SWM_GB300_SOR_BLOCKS
+  const int want = sor_env("SWM_GB300_SOR_BLOCKS");
+  sor_blocks(s, ns, want ? want : sms);
   SWM_CK(cudaMalloc((void **)&s->rows, (size_t)c->ny * sizeof(SorRow)));
   for (int col = 0; col < 2; col++) {
     SWM_CK(cudaMalloc((void **)&s->Bs[col], ns * 8));
@@ -521,6 +534,27 @@ int elsolv_sor_gpu_init(swm_gpu_ctx *c) {
 
 }  // extern "C"
 
+// One cooperative launch of niter iterations.  Where fewer blocks fit on the
+// GPU at once than there are (a context that is given part of the SMs), the
+// launch is refused and half as many blocks take the same cells.
+static int sor_batch(swm_gpu_ctx *c, double rJ, int niter) {
+  SorState *s = c->sor;
+  int nx = c->nx, ny = c->ny;
+  void *args[] = {s, &nx, &ny, &rJ, &niter};
+  for (;;) {
+    SWM_CK(cudaMemsetAsync(s->flags, 0, 2 * s->blocks * sizeof(unsigned), c->stream));
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_sor_batch, dim3(s->blocks), dim3(s->threads), args,
+                                                      0, c->stream);
+    if (e != cudaErrorCooperativeLaunchTooLarge || s->blocks == 1) {
+      SWM_CK(e);
+      c->launches++;
+      return SWM_GPU_OK;
+    }
+    cudaGetLastError();
+    sor_blocks(s, (size_t)s->W * c->ny, (s->blocks + 1) / 2);
+  }
+}
+
 // main_ElSolv_SOR on the device arrays s->B (right-hand side) and chi
 // (first guess in, solution out), natural layout; returns
 // SWM_GPU_ENOT_CONVERGED after max_count iterations
@@ -540,14 +574,12 @@ static int sor_solve_device(swm_gpu_ctx *c, double *chi, double eps, int first_g
   ctl.eps = eps;
   SWM_CK(cudaMemcpyAsync(s->ctl, &ctl, sizeof(SorCtl), cudaMemcpyHostToDevice, c->stream));
   double rJ = (double)(float)9.9999178e-1;  // default-real literal (ElSolv_SOR.f90:175)
-  int nx = c->nx, ny = c->ny;
-  // iterations of a batch: some tens of milliseconds at 4e10 cells a second
-  int batch = (int)std::min(4096., std::max(16., 1e9 / (double)c->n));
-  void *args[] = {s, &nx, &ny, &rJ, &batch};
+  // iterations of a batch: some tens of milliseconds at 4e10 cells a second, or SWM_GB300_SOR_BATCH
+  const int want = sor_env("SWM_GB300_SOR_BATCH");
+  const int batch = want ? std::min(want, max_count) : (int)std::min(4096., std::max(16., 1e9 / (double)c->n));
   for (int l = 1; l <= max_count; l += batch) {
-    SWM_CK(cudaMemsetAsync(s->flags, 0, 2 * s->blocks * sizeof(unsigned), c->stream));
-    SWM_CK(cudaLaunchCooperativeKernel((const void *)k_sor_batch, dim3(s->blocks), dim3(s->threads), args, 0, c->stream));
-    c->launches++;
+    const int rc = sor_batch(c, rJ, batch);
+    if (rc != SWM_GPU_OK) return rc;
     SWM_CK(cudaMemcpyAsync(&ctl, s->ctl, sizeof(SorCtl), cudaMemcpyDeviceToHost, c->stream));
     SWM_CK(cudaStreamSynchronize(c->stream));
     if (ctl.failed) {
