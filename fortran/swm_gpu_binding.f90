@@ -462,6 +462,11 @@ module swm_gpu_binding
       type(c_ptr), value :: chi
       type(c_ptr), value :: iterations
     end function swm_gpu_nondivergent
+    integer(c_int) function swm_gpu_check_sor_wait(ctx, limit_ms) bind(C)
+      import :: c_int, c_ptr
+      type(c_ptr), value :: ctx
+      integer(c_int), value :: limit_ms
+    end function swm_gpu_check_sor_wait
     integer(c_int) function swm_gpu_check_division(n, seed, mismatches) bind(C)
       import :: c_int, c_int64_t, c_ptr
       integer(c_int64_t), value :: n

@@ -314,7 +314,10 @@ int trc_gpu_get_field(swm_gpu_ctx *ctx, int tracer, int field, double *host_out)
 /* ---- red-black SOR (ElSolv_SOR.f90) ---- */
 int elsolv_sor_gpu_init(swm_gpu_ctx *ctx);   /* init_ElSolv_SOR (:44-66) */
 /* main_ElSolv_SOR (:150-222); returns SWM_GPU_ENOT_CONVERGED when max_count
-   sweeps did not bring the correction norm below eps */
+   sweeps did not bring the correction norm below eps.  Its blocks wait for
+   one another within a (cooperative) launch; a wait that has not ended after
+   2 s, because blocks were preempted for that long, ends the solve with
+   SWM_GPU_EDEVICE and chi as it came */
 int elsolv_sor_gpu_solve(swm_gpu_ctx *ctx, const double *B, double *chi, double eps, int first_guess,
                          int *iterations, double *anorm);
 /* computeNonDivergentFlowField (calc_lib.f90:548-590) of the current model
@@ -322,9 +325,15 @@ int elsolv_sor_gpu_solve(swm_gpu_ctx *ctx, const double *B, double *chi, double 
    for chi (kept on the device between calls, like calc_lib::chi;
    first_guess = itt == 1; eps = EPS of calc_lib.h, 1e-4), computeGradient
    (:638-648); u_nd = u - d chi / (A cos dLambda), v_nd = v - d chi / (A
-   dTheta).  Outputs may be NULL. */
+   dTheta).  Outputs may be NULL.  Statuses as elsolv_sor_gpu_solve; after
+   SWM_GPU_EDEVICE the outputs are not written. */
 int swm_gpu_nondivergent(swm_gpu_ctx *ctx, int first_guess, double eps, double *u_nd, double *v_nd, double *chi,
                          int *iterations);
+/* self-check of the solver's bounded waits: one launch whose blocks also wait
+   for a block that there is not, for at most limit_ms (1 to 1000); returns
+   SWM_GPU_EDEVICE when the waits ended as they should.  The context and chi
+   of swm_gpu_nondivergent stay as they were. */
+int swm_gpu_check_sor_wait(swm_gpu_ctx *ctx, int limit_ms);
 /* Self-check of the division by a fixed divisor that the SOR half-sweep
    and the plain path use (a / b formed from the reciprocal of b by two
    Markstein corrections, other numerators by exact branches) against the

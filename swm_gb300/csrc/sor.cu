@@ -89,6 +89,8 @@ struct SorState {
   int W = 0;                   // split row length
   unsigned span = 0;           // cells of a colour per block
   int blocks = 0, threads = 0; // of a batch; the last warp adds the norms
+  unsigned parties = 0;        // blocks that wait for one another
+  unsigned long long wait_ns = 0;  // a wait that has not ended after this gives up
 };
 
 constexpr int SOR_CELL_THREADS = 480;  // most threads of a block that own cells
@@ -96,7 +98,7 @@ constexpr int SOR_CELLS = 4;           // cells whose loads a thread has in flig
 // kept norms: a block that starts adding iteration l + 3's has decided l + 1,
 // for which every block has started l + 2 and so decided l
 constexpr int SOR_PART = 4;            // (also the relaxation factors' ring)
-constexpr unsigned long long SOR_WAIT_NS = 2000000000ull;  // a wait that has not ended after 2 s
+constexpr unsigned long long SOR_WAIT_NS = 2000000000ull;  // 2 s
 
 namespace swm {
 
@@ -151,7 +153,7 @@ __global__ void k_sor_mask(Dev d, uint8_t *__restrict__ ms, int W, int col) {
 // thread's did (ctl->failed).
 // SLEEP: nanoseconds between looks, for waits that are not urgent.
 template <int SLEEP = 0, typename F>
-__device__ __forceinline__ bool sor_wait(SorCtl *ctl, F ready) {
+__device__ __forceinline__ bool sor_wait(SorCtl *ctl, unsigned long long limit, F ready) {
   unsigned long long t0 = 0;
   for (unsigned spins = 1;; spins++) {
     if (ready()) return true;
@@ -160,7 +162,7 @@ __device__ __forceinline__ bool sor_wait(SorCtl *ctl, F ready) {
       unsigned long long t;
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
       if (t0 == 0) t0 = t;
-      if (t - t0 > SOR_WAIT_NS) atomicExch(&ctl->failed, 1u);
+      if (t - t0 > limit) atomicExch(&ctl->failed, 1u);
       if (*(volatile unsigned *)&ctl->failed) return false;
     }
   }
@@ -192,7 +194,7 @@ __global__ void __launch_bounds__(SOR_CELL_THREADS + 32, 1) k_sor_batch(SorState
   __shared__ int go, fail;
   const int l0 = ctl->l, lend = min(l0 + niter - 1, ctl->max_count);
   if (ctl->done || ctl->failed || l0 > lend) return;  // the same in every block: nobody has written yet
-  const unsigned W = s.W, ns = W * (unsigned)ny, G = gridDim.x, blk = blockIdx.x, span = s.span;
+  const unsigned W = s.W, ns = W * (unsigned)ny, G = s.parties, blk = blockIdx.x, span = s.span;
   const unsigned q0 = blk * span, q1 = min(q0 + span, ns);
   const unsigned tid = threadIdx.x, T = blockDim.x - 32;  // threads that own cells
   const double eps = ctl->eps;
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(SOR_CELL_THREADS + 32, 1) k_sor_batch(SorState
     int l = l0;
     bool ok = true, met = false;
     for (; l <= lend && !met; l++) {
-      ok = sor_wait(ctl, [&]() { return swept >= l; });
+      ok = sor_wait(ctl, s.wait_ns, [&]() { return swept >= l; });
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       __threadfence_block();
@@ -239,7 +241,7 @@ __global__ void __launch_bounds__(SOR_CELL_THREADS + 32, 1) k_sor_batch(SorState
       }
       __syncwarp();
       for (unsigned b = lane; b < G && ok; b += 32)
-        ok = sor_wait<20>(ctl, [&]() { return sor_flag(stored + b) >= (unsigned)(l - l0) + 1u; });
+        ok = sor_wait<20>(ctl, s.wait_ns, [&]() { return sor_flag(stored + b) >= (unsigned)(l - l0) + 1u; });
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       v = 0.;
@@ -282,10 +284,10 @@ __global__ void __launch_bounds__(SOR_CELL_THREADS + 32, 1) k_sor_batch(SorState
       if (h)
         for (unsigned t = tid; t < near && ok; t += T) {
           const unsigned b = (first + t) % G;
-          if (b != blk) ok = sor_wait(ctl, [&]() { return sor_flag(s.flags + b) >= h; });
+          if (b != blk) ok = sor_wait(ctl, s.wait_ns, [&]() { return sor_flag(s.flags + b) >= h; });
         }
       if (tid == 0 && col == 0) {
-        ok = ok && sor_wait(ctl, [&]() { return decided >= l - 2; });
+        ok = ok && sor_wait(ctl, s.wait_ns, [&]() { return decided >= l - 2; });
         __threadfence_block();
         go = stop > l - 2;
       }
@@ -483,6 +485,7 @@ static void sor_blocks(SorState *s, size_t ns, int blocks) {
   s->span = (unsigned)std::max<size_t>(32, (ns + blocks - 1) / blocks);
   s->blocks = (int)((ns + s->span - 1) / s->span);
   s->threads = (int)std::min<size_t>(SOR_CELL_THREADS, ((size_t)s->span + 31) / 32 * 32) + 32;
+  s->parties = (unsigned)s->blocks;
 }
 
 // a whole number from the environment, 0 when unset or not positive
@@ -507,6 +510,7 @@ int elsolv_sor_gpu_init(swm_gpu_ctx *c) {
   // one block per SM, or SWM_GB300_SOR_BLOCKS
   const int want = sor_env("SWM_GB300_SOR_BLOCKS");
   sor_blocks(s, ns, want ? want : sms);
+  s->wait_ns = SOR_WAIT_NS;
   SWM_CK(cudaMalloc((void **)&s->rows, (size_t)c->ny * sizeof(SorRow)));
   for (int col = 0; col < 2; col++) {
     SWM_CK(cudaMalloc((void **)&s->Bs[col], ns * 8));
@@ -517,9 +521,9 @@ int elsolv_sor_gpu_init(swm_gpu_ctx *c) {
   SWM_CK(cudaMalloc((void **)&s->chi, n * 8));
   SWM_CK(cudaMalloc((void **)&s->chi_io, n * 8));
   SWM_CK(cudaMalloc((void **)&s->B, n * 8));
-  SWM_CK(cudaMalloc((void **)&s->partial, (size_t)SOR_PART * s->blocks * 8));
+  SWM_CK(cudaMalloc((void **)&s->partial, (size_t)SOR_PART * (s->blocks + 1) * 8));
   SWM_CK(cudaMalloc((void **)&s->ctl, sizeof(SorCtl)));
-  SWM_CK(cudaMalloc((void **)&s->flags, 2 * s->blocks * sizeof(unsigned)));
+  SWM_CK(cudaMalloc((void **)&s->flags, 2 * (s->blocks + 1) * sizeof(unsigned)));
   SWM_CK(cudaMemsetAsync(s->ctl, 0, sizeof(SorCtl), c->stream));
   SWM_CK(cudaMemsetAsync(s->chi, 0, n * 8, c->stream));  // calc_lib::chi starts at 0
   const Dev d = c->dev();
@@ -542,7 +546,7 @@ static int sor_batch(swm_gpu_ctx *c, double rJ, int niter) {
   int nx = c->nx, ny = c->ny;
   void *args[] = {s, &nx, &ny, &rJ, &niter};
   for (;;) {
-    SWM_CK(cudaMemsetAsync(s->flags, 0, 2 * s->blocks * sizeof(unsigned), c->stream));
+    SWM_CK(cudaMemsetAsync(s->flags, 0, 2 * s->parties * sizeof(unsigned), c->stream));
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_sor_batch, dim3(s->blocks), dim3(s->threads), args,
                                                       0, c->stream);
     if (e != cudaErrorCooperativeLaunchTooLarge || s->blocks == 1) {
@@ -615,6 +619,20 @@ int elsolv_sor_gpu_solve(swm_gpu_ctx *c, const double *B, double *chi, double ep
   int rc = sor_solve_device(c, s->chi_io, eps, first_guess, iters, anorm);
   SWM_CK(cudaMemcpyAsync(chi, s->chi_io, n * 8, cudaMemcpyDeviceToHost, c->stream));
   SWM_CK(cudaStreamSynchronize(c->stream));
+  return rc;
+}
+
+int swm_gpu_check_sor_wait(swm_gpu_ctx *c, int limit_ms) {
+  SWM_ON_DEVICE(c ? c->device : -1);
+  SWM_REQUIRE(c && c->sor && limit_ms > 0 && limit_ms <= 1000, "swm_gpu_check_sor_wait: bad arguments");
+  SorState *s = c->sor;
+  SWM_CK(cudaMemsetAsync(s->chi_io, 0, c->n * 8, c->stream));
+  SWM_CK(cudaMemsetAsync(s->B, 0, c->n * 8, c->stream));
+  s->parties = (unsigned)s->blocks + 1;  // the last one is no block
+  s->wait_ns = 1000000ull * (unsigned)limit_ms;
+  const int rc = sor_solve_device(c, s->chi_io, 1e-300, 0, nullptr, nullptr);
+  s->parties = (unsigned)s->blocks;
+  s->wait_ns = SOR_WAIT_NS;
   return rc;
 }
 

@@ -74,3 +74,19 @@ def test_more_blocks_than_fit(monkeypatch):
         g.close()
     for x, n, _ in out[1:]:
         assert n == out[0][1] and np.array_equal(x, out[0][0])
+
+
+@pytest.mark.parametrize('shape,blocks', [((64, 48), 0), ((200, 100), 3)])   # every block a neighbour, or two of them
+def test_a_wait_that_runs_out(shape, blocks, monkeypatch):
+    """Blocks that wait for one that never comes give up and say so; the
+    context solves as before afterwards."""
+    case, o, B = problem(shape)
+    want, its, _ = o.sor_solve(B, np.zeros_like(B), 1e-40, False)
+    g = gpu(case, monkeypatch, blocks, 0)
+    assert g.L.swm_gpu_check_sor_wait(g.ctx, 20) == 5
+    assert b'waited too long' in g.L.swm_gpu_last_error()
+    for limit in (0, -1, 1001):
+        assert g.L.swm_gpu_check_sor_wait(g.ctx, limit) == 1
+    got, n, _ = g.sor_solve(B, np.zeros_like(B), 1e-40, False)
+    assert n == its and np.array_equal(got, want)
+    g.close()
