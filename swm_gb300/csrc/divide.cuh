@@ -108,13 +108,4 @@ __device__ __forceinline__ double div_fixed(double a, const FixedDiv &d) {
   return __ddiv_rn(a, d.b);
 }
 
-// the host's check of a divisor for div_fast
-inline bool div_host_range(double x) {
-  if (!(x - x == 0.) || x == 0.) return false;  // infinite, NaN or zero
-  int e = 0;
-  const double m = __builtin_frexp(x < 0 ? -x : x, &e);
-  (void)m;
-  return e - 1 >= -500 && e - 1 <= 500;
-}
-
 }  // namespace swm

@@ -38,11 +38,6 @@ __device__ __forceinline__ double ip2_noland(const double *v, const int8_t *m, s
   double w = inv_count(m[k1] + m[k2]);
   return mw(m[k1], w) * v[k1] + mw(m[k2], w) * v[k2];
 }
-__device__ __forceinline__ double ip4_noland(const double *v, const int8_t *m, size_t k1, size_t k2,
-                                             size_t k3, size_t k4) {
-  double w = inv_count(m[k1] + m[k2] + m[k3] + m[k4]);
-  return mw(m[k1], w) * v[k1] + mw(m[k2], w) * v[k2] + mw(m[k3], w) * v[k3] + mw(m[k4], w) * v[k4];
-}
 __device__ __forceinline__ double ip2(const double *v, size_t k1, size_t k2) { return .5 * v[k1] + .5 * v[k2]; }
 __device__ __forceinline__ double ip4(const double *v, size_t k1, size_t k2, size_t k3, size_t k4) {
   return .25 * v[k1] + .25 * v[k2] + .25 * v[k3] + .25 * v[k4];
@@ -59,7 +54,7 @@ __device__ __forceinline__ bool scalable(double x) {
 __device__ __forceinline__ bool is_one(double a) { return __double_as_longlong(a) == 0x3ff0000000000000ll; }
 __device__ __forceinline__ bool zero2(double a, double b) { return ((__double_as_longlong(a) | __double_as_longlong(b)) << 1) == 0; }
 
-// ip4_noland / ip2_noland of values in hand, 0 where the point is land
+// the mask-weighted means of four and of two values in hand, 0 where the point is land
 __device__ __forceinline__ double mean4_noland(double a, double b, double c, double d, int n, int na, int nb, int nc,
                                                int nd) {
   const double s = ((a + b) + c) + d, w = inv_count(n);
@@ -393,7 +388,6 @@ __global__ void __launch_bounds__(256) k_plain_diag(Dev d, DiagJobs w) {
 }
 
 struct ABCoef {
-  double c[3];
   double dtc[3];  // dt * c[t], the product the reference forms first (host, the same rounding)
   int tstep;
 };
@@ -803,10 +797,7 @@ int plain_step(swm_gpu_ctx *c, int64_t itt) {
   ab.tstep = (int)(itt < 3 ? itt : 3);
   const double chi = c->cfg.ab_chi;
   double tab[4][3] = {{0, 0, 0}, {1., 0, 0}, {-0.5 - chi, 1.5 + chi, 0}, {5. / 12., -16. / 12., 23. / 12.}};
-  for (int q = 0; q < 3; q++) {
-    ab.c[q] = tab[ab.tstep][q];
-    ab.dtc[q] = c->cfg.dt * ab.c[q];
-  }
+  for (int q = 0; q < 3; q++) ab.dtc[q] = c->cfg.dt * tab[ab.tstep][q];
   LAUNCH(k_plain_step, d, tuv, ab);
   SWM_CK(cudaGetLastError());
   c->stress_ready = false;
