@@ -97,16 +97,15 @@ swm::Dev swm_gpu_ctx::dev() const {
   return d;
 }
 
-// allocations are zeroed on the context's stream, so that later kernels on
-// that (non-blocking) stream are ordered after the zeroing
-static cudaStream_t g_alloc_stream = nullptr;
-static int dalloc(double **p, size_t n) {
+// allocations are zeroed on the context's stream, so that later kernels and
+// copies on that (non-blocking) stream are ordered after the zeroing
+static int dalloc(swm_gpu_ctx *c, double **p, size_t n) {
   cudaError_t e = cudaMalloc((void **)p, n * sizeof(double));
   if (e != cudaSuccess) {
     set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
     return SWM_GPU_ENOMEM;
   }
-  e = cudaMemsetAsync(*p, 0, n * sizeof(double), g_alloc_stream);
+  e = cudaMemsetAsync(*p, 0, n * sizeof(double), c->stream);
   if (e != cudaSuccess) {
     set_error(std::string("cudaMemset: ") + cudaGetErrorString(e));
     return SWM_GPU_ECUDA;
@@ -226,41 +225,40 @@ int swm_gpu_domain(swm_gpu_ctx *c, const double *H, const int8_t *Hmiss) {
   SWM_ON_DEVICE(c ? c->device : -1);
   SWM_REQUIRE(c && c->stage == 0, "swm_gpu_domain: call once, first");
   TRY(host_domain(c, H, Hmiss));
-  g_alloc_stream = c->stream;
   size_t n = c->n;
   int ny = c->ny;
   const HostGrid &g = c->hg;
   for (int q = 0; q < 4; q++) {
     SWM_CK(cudaMalloc((void **)&c->d_ocean[q], n));
-    SWM_CK(cudaMemcpy(c->d_ocean[q], g.ocean[q].data(), n, cudaMemcpyHostToDevice));
-    TRY(dalloc(&c->d_cos[q], ny));
-    TRY(dalloc(&c->d_tan[q], ny));
-    TRY(dalloc(&c->d_f[q], ny));
-    TRY(dalloc(&c->d_lat[q], ny));
-    TRY(dalloc(&c->d_H[q], n));
-    SWM_CK(cudaMemcpy(c->d_cos[q], g.cosl[q].data(), ny * 8, cudaMemcpyHostToDevice));
-    SWM_CK(cudaMemcpy(c->d_tan[q], g.tanl[q].data(), ny * 8, cudaMemcpyHostToDevice));
-    SWM_CK(cudaMemcpy(c->d_f[q], g.f[q].data(), ny * 8, cudaMemcpyHostToDevice));
-    SWM_CK(cudaMemcpy(c->d_lat[q], g.lat[q].data(), ny * 8, cudaMemcpyHostToDevice));
-    SWM_CK(cudaMemcpy(c->d_H[q], g.H[q].data(), n * 8, cudaMemcpyHostToDevice));
+    SWM_CK(upload(c->d_ocean[q], g.ocean[q].data(), n, c->stream));
+    TRY(dalloc(c, &c->d_cos[q], ny));
+    TRY(dalloc(c, &c->d_tan[q], ny));
+    TRY(dalloc(c, &c->d_f[q], ny));
+    TRY(dalloc(c, &c->d_lat[q], ny));
+    TRY(dalloc(c, &c->d_H[q], n));
+    SWM_CK(upload(c->d_cos[q], g.cosl[q].data(), ny * 8, c->stream));
+    SWM_CK(upload(c->d_tan[q], g.tanl[q].data(), ny * 8, c->stream));
+    SWM_CK(upload(c->d_f[q], g.f[q].data(), ny * 8, c->stream));
+    SWM_CK(upload(c->d_lat[q], g.lat[q].data(), ny * 8, c->stream));
+    SWM_CK(upload(c->d_H[q], g.H[q].data(), n * 8, c->stream));
   }
   for (int q = 0; q < 2; q++) {
-    TRY(dalloc(&c->u[q], n)); TRY(dalloc(&c->v[q], n)); TRY(dalloc(&c->eta[q], n));
+    TRY(dalloc(c, &c->u[q], n)); TRY(dalloc(c, &c->v[q], n)); TRY(dalloc(c, &c->eta[q], n));
   }
   for (int q = 0; q < 3; q++) {
-    TRY(dalloc(&c->Gu[q], n)); TRY(dalloc(&c->Gv[q], n)); TRY(dalloc(&c->Ge[q], n));
-    TRY(dalloc(&c->impl[q], n)); TRY(dalloc(&c->glin[q], n)); TRY(dalloc(&c->F[q], n)); TRY(dalloc(&c->Fc[q], n));
+    TRY(dalloc(c, &c->Gu[q], n)); TRY(dalloc(c, &c->Gv[q], n)); TRY(dalloc(c, &c->Ge[q], n));
+    TRY(dalloc(c, &c->impl[q], n)); TRY(dalloc(c, &c->glin[q], n)); TRY(dalloc(c, &c->F[q], n)); TRY(dalloc(c, &c->Fc[q], n));
   }
-  for (int q = 0; q < 2; q++) TRY(dalloc(&c->gsq[q], n));
-  TRY(dalloc(&c->edens, n)); TRY(dalloc(&c->pot, n)); TRY(dalloc(&c->zeta, n));
-  TRY(dalloc(&c->mu, n)); TRY(dalloc(&c->mv, n));
-  TRY(dalloc(&c->pll, n)); TRY(dalloc(&c->plt, n)); TRY(dalloc(&c->lmu, n)); TRY(dalloc(&c->lmv, n));
-  TRY(dalloc(&c->ubs, n)); TRY(dalloc(&c->vbs, n)); TRY(dalloc(&c->zbs, n));
+  for (int q = 0; q < 2; q++) TRY(dalloc(c, &c->gsq[q], n));
+  TRY(dalloc(c, &c->edens, n)); TRY(dalloc(c, &c->pot, n)); TRY(dalloc(c, &c->zeta, n));
+  TRY(dalloc(c, &c->mu, n)); TRY(dalloc(c, &c->mv, n));
+  TRY(dalloc(c, &c->pll, n)); TRY(dalloc(c, &c->plt, n)); TRY(dalloc(c, &c->lmu, n)); TRY(dalloc(c, &c->lmv, n));
+  TRY(dalloc(c, &c->ubs, n)); TRY(dalloc(c, &c->vbs, n)); TRY(dalloc(c, &c->zbs, n));
   if (c->cfg.mode == SWM_MODE_NONLINEAR) {
-    for (int q = 0; q < 4; q++) { TRY(dalloc(&c->Dbuf[q], n)); TRY(plain_fill(c, c->Dbuf[q], 1.)); }
+    for (int q = 0; q < 4; q++) { TRY(dalloc(c, &c->Dbuf[q], n)); TRY(plain_fill(c, c->Dbuf[q], 1.)); }
   }
   if (c->cfg.lateral_mixing && c->cfg.mixing_kind == SWM_MIX_BIHARMONIC) {
-    for (int q = 0; q < 4; q++) TRY(dalloc(&c->bh[q], n));
+    for (int q = 0; q < 4; q++) TRY(dalloc(c, &c->bh[q], n));
   }
   for (int q = 0; q < 3; q++) TRY(plain_fill(c, c->impl[q], 1.));
   c->n0 = 0;
@@ -329,9 +327,8 @@ int swm_gpu_add_stream(swm_gpu_ctx *c, int type, int comp, double omega, int is_
   if (type == SWM_FRC_OSC) s.is_const = 0;
   else if (type == SWM_FRC_WIND && c->cfg.mode == SWM_MODE_NONLINEAR) s.is_const = 0;
   else s.is_const = is_const ? 1 : 0;
-  g_alloc_stream = c->stream;
-  TRY(dalloc(&s.d1, c->n));
-  TRY(dalloc(&s.d2, c->n));
+  TRY(dalloc(c, &s.d1, c->n));
+  TRY(dalloc(c, &s.d2, c->n));
   if (d1) TRY(h2d(c, s.d1, d1, c->n));
   if (d2) TRY(h2d(c, s.d2, d2, c->n));
   c->streams.push_back(s);

@@ -207,6 +207,14 @@ void host_damping_add(swm_gpu_ctx *c, int term, int type, double value, double s
                       double sl_cutoff, int loc, const double *file_data);
 void host_damping_finish(swm_gpu_ctx *c);
 
+// host data -> device, complete on return, on the stream whose kernels read it:
+// a copy on the default stream is ordered neither with the zeroing of its
+// destination nor with the kernels that follow on a context's own stream
+inline cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 // plain.cu
 int plain_diagnostics(swm_gpu_ctx *c, int64_t itt);
 int plain_step(swm_gpu_ctx *c, int64_t itt);

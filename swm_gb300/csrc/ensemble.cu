@@ -278,7 +278,7 @@ int ens_monitor_setup(swm_gpu_ensemble *e) {
   for (int t = 0; t < e->ntiles; t++) tiles_of[fill[e->htiles[t].x]++] = t;
   auto up = [&](void **dst, const void *src, size_t bytes) {
     if (cudaMalloc(dst, bytes) != cudaSuccess) return SWM_GPU_ENOMEM;
-    if (src && cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return SWM_GPU_ECUDA;
+    if (src && upload(*dst, src, bytes, e->stream) != cudaSuccess) return SWM_GPU_ECUDA;
     return SWM_GPU_OK;
   };
   int rc = SWM_GPU_OK;
@@ -436,7 +436,7 @@ int swm_gpu_ensemble_create(swm_gpu_ctx *const *members, int n, swm_gpu_ensemble
     maxn = std::max(maxn, lists[r].size());
   }
   if (cudaMalloc((void **)&e->tab, tab.size() * sizeof(P32)) != cudaSuccess ||
-      cudaMemcpy(e->tab, tab.data(), tab.size() * sizeof(P32), cudaMemcpyHostToDevice) != cudaSuccess ||
+      upload(e->tab, tab.data(), tab.size() * sizeof(P32), e->stream) != cudaSuccess ||
       cudaMalloc((void **)&e->next, ENS_PHASES * sizeof(int)) != cudaSuccess ||
       cudaMalloc((void **)&e->d_int, n * sizeof(EnsInt)) != cudaSuccess ||
       cudaMalloc((void **)&e->d_out, 3 * (size_t)n * sizeof(double)) != cudaSuccess) {

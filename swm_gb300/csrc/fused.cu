@@ -91,9 +91,9 @@ static int upload_t(swm_gpu_ctx *c, bool f32, const double *host, size_t count, 
   if (f32) {
     std::vector<float> t(count);
     for (size_t q = 0; q < count; q++) t[q] = (float)host[q];
-    SWM_CK(cudaMemcpy(*dst, t.data(), count * 4, cudaMemcpyHostToDevice));
+    SWM_CK(upload(*dst, t.data(), count * 4, c->stream));
   } else {
-    SWM_CK(cudaMemcpy(*dst, host, count * 8, cudaMemcpyHostToDevice));
+    SWM_CK(upload(*dst, host, count * 8, c->stream));
   }
   return SWM_GPU_OK;
 }
@@ -128,7 +128,7 @@ int fused_prepare(swm_gpu_ctx *c) {
   for (size_t k = 0; k < n; k++)
     mc[k] = (uint8_t)(g.ocean[GH][k] | (g.ocean[GU][k] << 1) | (g.ocean[GV][k] << 2) | (g.ocean[GE][k] << 3));
   FTRY(dmalloc((void **)&f->mc, n));
-  SWM_CK(cudaMemcpy(f->mc, mc.data(), n, cudaMemcpyHostToDevice));
+  SWM_CK(upload(f->mc, mc.data(), n, c->stream));
   // per-row metric factors, from the FP64 grid
   if (!f32) {
     const std::vector<double> rows = fused64_rows(c);
@@ -207,7 +207,7 @@ int fused_prepare(swm_gpu_ctx *c) {
   if (f32) {
     const std::vector<float> rec = fp32c_records(c);
     FTRY(dmalloc(&f->rows32c, rec.size() * sizeof(float)));
-    SWM_CK(cudaMemcpy(f->rows32c, rec.data(), rec.size() * sizeof(float), cudaMemcpyHostToDevice));
+    SWM_CK(upload(f->rows32c, rec.data(), rec.size() * sizeof(float), c->stream));
     // mask word with the x-neighbours' bits (bits 4-7: i-1, 8-11: i+1)
     std::vector<uint16_t> m16(n);
     int nx = c->nx;
@@ -218,7 +218,7 @@ int fused_prepare(swm_gpu_ctx *c) {
         m16[k] = (uint16_t)(mc[k] | (mc[kl] << 4) | (mc[kr] << 8));
       }
     FTRY(dmalloc((void **)&f->mask16, n * 2));
-    SWM_CK(cudaMemcpy(f->mask16, m16.data(), n * 2, cudaMemcpyHostToDevice));
+    SWM_CK(upload(f->mask16, m16.data(), n * 2, c->stream));
     f->m16h = std::move(m16);
     // implicit damping as the removed fraction dt*gamma/(1 + dt*gamma)
     for (int q = 0; q < 3; q++) f->dp_s[q] = (f->impl_s[q] - 1.) / f->impl_s[q];
@@ -1212,10 +1212,10 @@ static int integrals_scratch(swm_gpu_ctx *c, IntegralScratch **out) {
     SWM_CK(cudaMalloc((void **)&S->partial, 3 * (size_t)INTEGRALS_MAX_BLOCKS * sizeof(double)));
     SWM_CK(cudaMalloc((void **)&S->out, 3 * sizeof(double)));
     SWM_CK(cudaMalloc((void **)&S->done, sizeof(unsigned)));
-    SWM_CK(cudaMemset(S->done, 0, sizeof(unsigned)));
+    SWM_CK(cudaMemsetAsync(S->done, 0, sizeof(unsigned), c->stream));
     SWM_CK(cudaMallocHost((void **)&S->host, 3 * sizeof(double)));
-    SWM_CK(cudaMemcpy(S->area, area.data(), 3 * ny * sizeof(double), cudaMemcpyHostToDevice));
-    SWM_CK(cudaMemcpy(S->pairs, pairs.data(), 3 * ny * sizeof(float2), cudaMemcpyHostToDevice));
+    SWM_CK(upload(S->area, area.data(), 3 * ny * sizeof(double), c->stream));
+    SWM_CK(upload(S->pairs, pairs.data(), 3 * ny * sizeof(float2), c->stream));
   }
   *out = S;
   return SWM_GPU_OK;

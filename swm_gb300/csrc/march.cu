@@ -1214,7 +1214,7 @@ static int upload_tiles(swm_gpu_ctx *c, const std::vector<int2> &t) {
   c->march_tiles = nullptr;
   c->march_blocks = 0;
   SWM_CK(cudaMalloc((void **)&c->march_tiles, t.size() * sizeof(int2)));
-  SWM_CK(cudaMemcpy(c->march_tiles, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice));
+  SWM_CK(upload(c->march_tiles, t.data(), t.size() * sizeof(int2), c->stream));
   c->march_blocks = (int)(t.size() / 4);
   return SWM_GPU_OK;
 }

@@ -250,11 +250,11 @@ int trc_gpu_add(swm_gpu_ctx *c, double kappa_h, double cons, double gamma_c, con
   SWM_CK(cudaMemcpyAsync(D.data(), d.D, n * 8, cudaMemcpyDeviceToHost, c->stream));
   SWM_CK(cudaStreamSynchronize(c->stream));
   for (size_t k = 0; k < n; k++) CH[k] = D[k] * Cv[k];
-  SWM_CK(cudaMemcpy(T.CH[0], CH.data(), n * 8, cudaMemcpyHostToDevice));
-  SWM_CK(cudaMemcpy(T.C, Cv.data(), n * 8, cudaMemcpyHostToDevice));
-  SWM_CK(cudaMemcpy(T.C0, C0v.data(), n * 8, cudaMemcpyHostToDevice));
-  SWM_CK(cudaMemcpy(T.gamma, gv.data(), n * 8, cudaMemcpyHostToDevice));
-  SWM_CK(cudaMemcpy(T.impl, impl.data(), n * 8, cudaMemcpyHostToDevice));
+  SWM_CK(upload(T.CH[0], CH.data(), n * 8, c->stream));
+  SWM_CK(upload(T.C, Cv.data(), n * 8, c->stream));
+  SWM_CK(upload(T.C0, C0v.data(), n * 8, c->stream));
+  SWM_CK(upload(T.gamma, gv.data(), n * 8, c->stream));
+  SWM_CK(upload(T.impl, impl.data(), n * 8, c->stream));
   if (c->cfg.path == SWM_PATH_FUSED_FP32C) TRY_T(trc32_add(c, CH, C0v, gv, impl, kappa_h));
   c->tracers.push_back(T);
   if (id) *id = (int)c->tracers.size() - 1;
