@@ -234,7 +234,7 @@ def double_gyre_line(args, rank, ws, steps, warmup, side=True):
     peak, kind = peaks()
     alg = BYTES_PER_POINT[args.path] * npts
     achieved = alg / (step_ms * 1e-3) / 1e9
-    kname = {'fused_fp32c': 'k_march', 'fused_fp64': 'k_fused'}.get(args.path)
+    kname = {'fused_fp32c': 'k_march', 'fused_fp64': 'k_f64'}.get(args.path)
     traffic = profiled_traffic('%s_double_gyre_%d.md' % (kname, cells)) if kname else None
     line['roofline'] = {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
                         'frac': achieved / peak, 'traffic': traffic, 'peak_kind': kind,

@@ -1,19 +1,21 @@
 // fused64.cu -- the FP64 step of the fused path: two kernels (diagnostics and
 // stress, then tendencies and update), four with biharmonic mixing.
 //
-// An FP64 warp instruction holds an SM's pipe for 19 cycles (9.75 ns), so the
-// step is bound by its FP64 operations and not by memory: one operation per
-// point of a 1025 x 1025 basin takes 2.1 us, 300 MB of traffic 45 us.  The
+// An FP64 warp instruction holds an SM's pipe for 18 to 19 cycles (8.9 ns), so
+// the step is bound by its FP64 operations and not by memory: one operation per
+// point of a 1025 x 1025 basin takes 1.9 us, 300 MB of traffic 45 us.  The
 // passes therefore form every quantity once per point and hand it on through
 // memory, instead of rebuilding it in the halo of a tile: a one-kernel step
 // whose tiles of 32 x 8 recompute two halo cells took 615 us there.  Masks are
 // selects, metric factors and mask cases per-row tables (of a difference, not
 // of its two terms, whose roundings would not cancel), stress and wind are
 // added before they are divided by the thickness, and a uniform implicit
-// damping factor divides as a fixed divisor (divide.cuh).  About 86 operations per point
-// (Laplacian), 104 (biharmonic).
+// damping factor divides as a fixed divisor (divide.cuh).  131 operations per
+// point (biharmonic, counted), three divisions among them.  Multiplying by a
+// thickness inverted once from the hardware's seed took 227 us a step, but
+// rounds twice.
 //
-// 1025 x 1025, biharmonic: 615 -> 252 us per step.
+// 1025 x 1025, biharmonic: 615 -> 252 us per step, the FP64 pipe's rate.
 //
 // Formulas: swm_nonlinear_timestep_module.f90:182-449 (diagnostics and
 // tendencies), swm_lateralmixing_module.f90:66-240 (stress), time_integration_

@@ -39,9 +39,10 @@
 //
 // One iteration, with a launch per colour and one-word reciprocals, and now:
 //   201 x 101 points      22.8 us ->   8.3 us  (waits and the FP64 latency chain)
-//   1025 x 769            47.0 us ->  32.3 us  (FP64 pipe 78 % busy; the 386 blocks of a
-//                                              colour left a last wave half empty)
-//   2049 x 2049            186 us ->   140 us  (FP64 pipe 95 % busy)
+//   1025 x 769            47.0 us ->  32.3 us  (its FP64 instructions take 78 % of that at the pipe's
+//                                              rate; the 386 blocks of a colour left a last wave
+//                                              half empty)
+//   2049 x 2049            186 us ->   140 us  (its FP64 instructions take 95 % of that)
 // at 9.75 ns per FP64 warp instruction and SM, measured (19 cycles).  480
 // threads of four cells in flight against 992 of one: 15.6 against 17.1 us at
 // 513 x 513, the same from 1025 x 769 on.
